@@ -10,14 +10,13 @@
 // go out as one cooperative grid walking a work list: each problem gets a
 // contiguous range of blocks (at most one block per SM in total, more blocks
 // for larger operators) and runs the same device function as the
-// single-problem kernel, with grid barriers replaced by barriers over its own
-// blocks.  Several problems then share the GPU inside one launch instead of
+// single-problem kernel, whose blocks exchange data through the problem's own
+// tagged words.  Several problems then share the GPU inside one launch instead of
 // queueing for it one multi-block grid at a time.
 //
-// Every block of a cooperative launch is resident, so a barrier over some of
-// its blocks always completes; each wait is still bounded (kSpinLimit polls),
-// after which the block raises the launch's error flag, every block of the
-// launch leaves at its next barrier, and the host reports EG_ERR_TIMEOUT.
+// Every block of a cooperative launch is resident, so the waits between a
+// problem's blocks always end; each is bounded all the same, and a solve that
+// gave up leaves its F_DONE at 0, which its caller reports as EG_ERR_TIMEOUT.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -25,124 +24,12 @@
 #include <mutex>
 #include <vector>
 
-#include "eg_arnoldi_body.cuh"
+#include "eg_arnoldi_batch.cuh"
+
+// k_gmres_batch<double> (eg_arnoldi_batch_f64.cu)
+const void* eg_gmres_batch_kernel_f64();
 
 namespace {
-
-constexpr int kMaxBatch = 128;               // problems per launch
-constexpr long long kSpinLimit = 1LL << 24;  // polls of one barrier wait
-
-// barrier over the nblk blocks of one problem of a batched launch; returns
-// false (in every thread of the block) once the launch's error flag is set
-struct SubBarrier {
-  unsigned int* count;  // arrivals at the current barrier
-  unsigned int* gen;    // generation, bumped by the last arrival
-  int* err;             // launch-wide flag: a wait gave up
-  int nblk;
-  int* s_ok;            // shared-memory broadcast slot
-  __device__ bool sync() {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int ok = 1;
-      if (nblk > 1) {
-        const unsigned int g = *(volatile unsigned int*)gen;
-        __threadfence();  // the block's writes before its arrival
-        if (atomicAdd(count, 1u) == (unsigned int)(nblk - 1)) {
-          *(volatile unsigned int*)count = 0u;
-          __threadfence();
-          atomicAdd(gen, 1u);
-        } else {
-          long long polls = 0;
-          while (*(volatile unsigned int*)gen == g) {
-            if (*(volatile int*)err) {
-              ok = 0;
-              break;
-            }
-            if (++polls > kSpinLimit) {
-              atomicExch(err, 1);
-              ok = 0;
-              break;
-            }
-            __nanosleep(64);
-          }
-        }
-        __threadfence();  // the other blocks' writes after the barrier
-      }
-      if (*(volatile int*)err) ok = 0;
-      *s_ok = ok;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-  }
-};
-
-// one work-list entry: the problem's kernel arguments (device copy), its
-// block range, its (dimension, block size) case and its chunk size
-struct BatchEntry {
-  const void* args;
-  int b0, nblk, kind, ec;
-};
-struct BatchList {
-  int n;
-  BatchEntry e[kMaxBatch];
-};
-
-// (dimension, element-block size) cases with a compiled body, the same set
-// as the single-problem launcher compiles for these dimensions (the block
-// size changes the order of the block-row sums); others run the generic body
-int kind_of(int dim, int n) {
-  if (dim == 2) {
-    switch (n) {
-      case 12: return 0;
-      case 24: return 1;
-      case 28: return 2;
-      case 40: return 3;
-      case 48: return 4;
-      case 60: return 5;
-      case 72: return 6;
-      default: return 7;
-    }
-  }
-  switch (n) {
-    case 30: return 8;
-    case 115: return 9;
-    default: return 10;
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(NT, 1) k_gmres_batch(BatchList list, unsigned int* bars, int* err) {
-  __shared__ GmresShared<T> sm;
-  __shared__ CoopArgs<T> sa;
-  __shared__ int s_k, s_nblk, s_b0, s_kind, s_ok;
-  if (threadIdx.x == 0) {
-    int k = 0;
-    while (k + 1 < list.n && (int)blockIdx.x >= list.e[k + 1].b0) ++k;
-    const BatchEntry en = list.e[k];
-    s_k = k;
-    s_nblk = en.nblk;
-    s_b0 = en.b0;
-    s_kind = en.kind;
-    sa = *reinterpret_cast<const CoopArgs<T>*>(en.args);
-    sa.ec = en.ec;
-  }
-  __syncthreads();
-  const int k = s_k, nblk = s_nblk, b = (int)blockIdx.x - s_b0;
-  SubBarrier bar{bars + 2 * k, bars + 2 * k + 1, err, nblk, &s_ok};
-  switch (s_kind) {
-    case 0: gmres_body<2, 12, T>(sa, b, nblk, bar, sm); break;
-    case 1: gmres_body<2, 24, T>(sa, b, nblk, bar, sm); break;
-    case 2: gmres_body<2, 28, T>(sa, b, nblk, bar, sm); break;
-    case 3: gmres_body<2, 40, T>(sa, b, nblk, bar, sm); break;
-    case 4: gmres_body<2, 48, T>(sa, b, nblk, bar, sm); break;
-    case 5: gmres_body<2, 60, T>(sa, b, nblk, bar, sm); break;
-    case 6: gmres_body<2, 72, T>(sa, b, nblk, bar, sm); break;
-    case 7: gmres_body<2, 0, T>(sa, b, nblk, bar, sm); break;
-    case 8: gmres_body<3, 30, T>(sa, b, nblk, bar, sm); break;
-    case 9: gmres_body<3, 115, T>(sa, b, nblk, bar, sm); break;
-    default: gmres_body<3, 0, T>(sa, b, nblk, bar, sm); break;
-  }
-}
 
 // ------------------------------------------------------------------ batcher
 struct Submission {
@@ -158,9 +45,6 @@ struct Batcher {
   std::chrono::steady_clock::time_point first;  // oldest pending hand-in
   bool launching = false;
   cudaStream_t stream = nullptr;  // the batched grids' stream
-  unsigned int* bars = nullptr;   // [kMaxBatch][2] barrier counters (device)
-  int* err = nullptr;             // device error flag
-  int* h_err = nullptr;           // pinned copy
   std::atomic<int> active{0};     // threads inside eg_newton_solve with a
                                   // multi-block Krylov solve
 };
@@ -176,9 +60,6 @@ std::atomic<long long> g_window_ns{50000};
 int ensure_batcher(Batcher& B) {
   if (B.stream) return EG_OK;
   cudaError_t e = cudaStreamCreateWithFlags(&B.stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&B.bars, sizeof(unsigned int) * 2 * kMaxBatch);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&B.err, sizeof(int));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&B.h_err, sizeof(int));
   if (e != cudaSuccess) return eg_cuda_fail(e, "GMRES batcher");
   return EG_OK;
 }
@@ -205,6 +86,25 @@ int wanted_blocks_sms(const eg_ls* ls, int sms) {
 }
 
 template <typename T>
+const void* batch_kernel() {
+  if constexpr (sizeof(T) == 8)
+    return eg_gmres_batch_kernel_f64();
+  else
+    return (const void*)k_gmres_batch<T>;
+}
+
+// a block of the batched kernel is resident with the largest shared memory
+// (asked of the runtime once per device; loads the kernel)
+template <typename T>
+bool batch_kernel_fits() {
+  return launch_fact(batch_kernel<T>(), 0, []() {
+    int per_sm = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_kernel<T>(), NT, kSmemBudget) ==
+               cudaSuccess && per_sm >= 1;
+  });
+}
+
+template <typename T>
 int launch_batch(Batcher& B, const std::vector<Submission*>& batch, int dev) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -216,43 +116,30 @@ int launch_batch(Batcher& B, const std::vector<Submission*>& batch, int dev) {
   size_t smem = 0;
   for (size_t i = 0; i < batch.size(); ++i) {
     const eg_ls* ls = batch[i]->ls;
-    const eg_mesh* m = ls->lo->mesh;
-    const int n = ls->lo->n;
-    const int epb = (m->E + nb[i] - 1) / nb[i];
-    const size_t elem_bytes = (size_t)n * sizeof(T);
-    int ec = (int)((40 * 1024) / elem_bytes);
-    ec = std::max(1, std::min(ec, epb));
-    smem = std::max(smem, (size_t)ec * elem_bytes);
-    list.e[i] = BatchEntry{ls->dargs, b0, nb[i], kind_of(m->dim, n), ec};
+    CoopArgs<T> a = *reinterpret_cast<const CoopArgs<T>*>(ls->hargs);
+    smem = std::max(smem, plan_smem(a, nb[i]));
+    list.e[i] = BatchEntry{ls->dargs, b0, nb[i], gmres_kind(ls), a.ec, a.fs_smem, a.ws, a.p0_smem, a.kv, a.er, a.ef0};
     b0 += nb[i];
   }
-  const void* fn = (const void*)k_gmres_batch<T>;
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, smem);
-  if (per_sm < 1 || b0 > sms * per_sm) {
+  const void* fn = batch_kernel<T>();
+  if (!batch_kernel_fits<T>() || b0 > sms) {
     eg_set_error("batched GMRES kernel cannot be resident");
     return EG_ERR_UNSUPPORTED;
   }
   std::lock_guard<std::mutex> lock(eg_coop_mutex(dev));
   for (Submission* s : batch) EG_CUDA(cudaStreamWaitEvent(B.stream, s->ls->ev_in, 0));
-  EG_CUDA(cudaMemsetAsync(B.bars, 0, sizeof(unsigned int) * 2 * list.n, B.stream));
-  EG_CUDA(cudaMemsetAsync(B.err, 0, sizeof(int), B.stream));
-  void* args[] = {&list, &B.bars, &B.err};
+  void* args[] = {&list};
   EG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(b0), dim3(NT), args, smem, B.stream));
-  EG_CUDA(cudaMemcpyAsync(B.h_err, B.err, sizeof(int), cudaMemcpyDeviceToHost, B.stream));
   EG_CUDA(cudaStreamSynchronize(B.stream));  // the grid has finished before the next one starts
   batch[0]->ls->lo->mesh->launches += 1;
-  if (*B.h_err) {
-    eg_set_error("batched GMRES: a barrier wait gave up");
-    return EG_ERR_TIMEOUT;
-  }
   return EG_OK;
 }
 
 template <typename T>
 int stage_args(eg_ls* ls) {
   eg_mesh* m = ls->lo->mesh;
+  const int rc = eg_gmres_tags(ls);
+  if (rc != EG_OK) return rc;
   if (!ls->dargs) {
     cudaError_t e = cudaMalloc(&ls->dargs, sizeof(CoopArgs<double>));
     if (e == cudaSuccess) e = cudaMallocHost(&ls->hargs, sizeof(CoopArgs<double>));
@@ -345,6 +232,20 @@ extern "C" int eg_set_gmres_batching(int32_t enable, double window_us) {
     return EG_ERR_INVALID;
   }
   g_window_ns.store((long long)(window_us * 1000.0));
+  if (enable) {
+    // the current device's batcher is set up here (stream, both batched
+    // kernels loaded), not by the first solve that is handed in
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) {
+      Batcher& B = batcher(dev);
+      std::lock_guard<std::mutex> lk(B.mu);
+      if (ensure_batcher(B) == EG_OK) {
+        batch_kernel_fits<float>();
+        batch_kernel_fits<double>();
+      }
+    }
+    cudaGetLastError();
+  }
   g_batching.store(enable);
   return EG_OK;
 }

@@ -629,8 +629,7 @@ int gmres_T(eg_ls* ls, eg_ls_stats* st, int transpose) {
   int fl[8] = {0, 0, 0, 0, ls->itermax, 0, 0, 0};
   EG_CUDA(cudaMemcpyAsync(ls->dscal, sc, sizeof(sc), cudaMemcpyHostToDevice, m->stream));
   EG_CUDA(cudaMemcpyAsync(ls->dflags, fl, sizeof(fl), cudaMemcpyHostToDevice, m->stream));
-  const bool coop = !transpose && eg_coop_usable(ls) && !m->capturing;
-  if (coop) {
+  if (eg_coop_usable(ls) && !m->capturing) {
     // the whole solve in one persistent launch
     const int rc = eg_gmres_coop(ls);
     if (rc != EG_OK) return rc;
@@ -641,6 +640,7 @@ int gmres_T(eg_ls* ls, eg_ls_stats* st, int transpose) {
     EG_CUDA(cudaStreamSynchronize(m->stream));
     std::memcpy(scal, ls->hh, sizeof(scal));
     std::memcpy(flags, ls->hh + 8, sizeof(flags));
+    if (!flags[F_DONE]) return eg_gmres_gave_up(ls);
     if (!std::isfinite(scal[S_BETA])) {
       eg_set_error("GMRES: non-finite residual");
       return EG_ERR_NONFINITE;

@@ -19,6 +19,7 @@ struct eg_lo {
   void* dF;        // [(I+B)][Nf][2][nv][nv] point flux Jacobians
   int32_t* spos;   // [F][Np]: stencil position of node j on face f, or -1
   int32_t* fside;  // [E][F]: coupling block (slot * 2 + side) of face f of e, or -1
+  int face_nodes;  // nodes on the stencil of some face
   void* xT;        // [ndof] operand in the operator precision
   void* yT;        // [ndof]
   double* xd;      // [ndof] FP64 staging
@@ -38,13 +39,18 @@ struct eg_ls {
   int m;           // restart length
   double reltol, abstol, dtol;
   int itermax;
-  void* V;         // [(m+1)][ndof]
+  void* V;         // [(m+1)][ndof] (stream path), or (m+2) vectors of the persistent
+                   // solve, block-local (eg_basis_values)
   void* w;         // [ndof]
   void* z;         // [ndof]
-  void* cfs;       // [I][2][nb] coupling products of each face side (persistent Arnoldi)
+  void* G;         // [E][n+1][F nbp] pushed operators of the persistent solve (dense
+                   // faces; null otherwise, or when there is no memory for them)
+  void* cfs;       // [I][2][nbp] tagged coupling products of each face side (persistent solve)
+  void* tpart;     // tagged partial sums and sums (persistent solve)
+  int64_t tags;    // bound on the tags used since they were last reset
   void* xT;        // [ndof]
   void* bT;        // [ndof]
-  void* part;      // [nblk][m+2] partial sums (operator precision)
+  void* part;      // [nblk][m+2][2] partial sums (operator precision, stream path)
   void* h;         // [m+2] device Hessenberg column (operator precision)
   double* hh;      // pinned host copy [m+2]
   void* y;         // [m+1] device least-squares solution
@@ -75,7 +81,9 @@ struct eg_ls {
 };
 void eg_gmres_release(eg_ls* ls);
 // slots of the device GMRES state: dflags[] and dscal[]
-enum { F_DONE = 0, F_JDONE = 1, F_ITS = 2, F_CONV = 3, F_ITERMAX = 4, F_REORTH = 5, F_CYCLES = 6, F_NREORTH = 7 };
+// (F_TAGS: two words, the last push and reduction tags of the persistent solve)
+enum { F_DONE = 0, F_JDONE = 1, F_ITS = 2, F_CONV = 3, F_ITERMAX = 4, F_REORTH = 5, F_CYCLES = 6, F_NREORTH = 7,
+       F_TAGS = 12 };
 enum { S_TOL = 0, S_RESID = 1, S_BETA = 2, S_BNORM = 3, S_RELTOL = 4, S_ABSTOL = 5, S_BETA0 = 6 };
 // the whole GMRES solve as one persistent cooperative kernel (eg_arnoldi.cu)
 #define EG_COOP_MAX_BLOCKS 1024
@@ -87,16 +95,27 @@ enum { S_TOL = 0, S_RESID = 1, S_BETA = 2, S_BNORM = 3, S_RELTOL = 4, S_ABSTOL =
 #endif
 // blocks of the stream GMRES path's reduction kernels (4 per SM)
 #define EG_GMRES_STREAM_BLOCKS 608
-// partial-sum slots of a GMRES(m) solver: the stream path's [blocks][m+2][2]
-// or the persistent kernel's [4][blocks][33], whichever is larger
-inline size_t eg_gmres_partials(int m) {
-  const size_t a = (size_t)EG_GMRES_STREAM_BLOCKS * (m + 2) * 2, b = (size_t)4 * EG_COOP_MAX_BLOCKS * 33;
-  return a > b ? a : b;
+// partial-sum slots of a GMRES(m) solver's stream path
+inline size_t eg_gmres_partials(int m) { return (size_t)EG_GMRES_STREAM_BLOCKS * (m + 2) * 2; }
+// rows of a face side in the persistent solve: nb padded to 16-byte units
+__host__ __device__ inline int eg_face_rows(int nb) { return (nb + 3) & ~3; }
+// values of the Krylov basis (and w): each block's rows are padded to 4
+inline size_t eg_basis_values(int m, int64_t N) { return (size_t)(m + 2) * ((size_t)N + 4 * (EG_COOP_MAX_BLOCKS + 1)); }
+// bytes of the persistent solve's buffers, es bytes per value: pushed
+// operators (dense faces), tagged face products, tagged partial sums
+inline size_t eg_push_operator_bytes(size_t E, size_t n, size_t F, int nb, size_t es) {
+  return es * E * (n + 1) * F * eg_face_rows(nb);
 }
+inline size_t eg_face_tag_bytes(size_t I, int nb, size_t es) { return 2 * es * I * 2 * eg_face_rows(nb); }
+inline size_t eg_part_tag_bytes(size_t es) { return 2 * es * 2 * 33 * (EG_COOP_MAX_BLOCKS + 16); }
+// before each persistent solve: reset the tagged buffers (on the mesh stream)
+// when the 32-bit tags could run out; `force` after a solve that gave up
+int eg_gmres_tags(eg_ls* ls, bool force = false);
+// a persistent solve ended without F_DONE: a wait between its blocks ran out.
+// Resets the tagged buffers and returns EG_ERR_TIMEOUT.
+int eg_gmres_gave_up(eg_ls* ls);
 int eg_gmres_coop(eg_ls* ls);
-// the persistent solve of a small system by one cluster of C blocks
-// (EG_ERR_UNSUPPORTED when no such cluster can be placed)
-int eg_gmres_cluster(eg_ls* ls, int C);
+int eg_gmres_launch_f64(eg_ls* ls);  // its FP64 launches (eg_arnoldi_f64.cu)
 // one cooperative GMRES grid at a time per device (held across launch and
 // completion of multi-block grids, single or batched)
 std::mutex& eg_coop_mutex(int dev);

@@ -750,6 +750,12 @@ extern "C" int eg_lo_create(eg_mesh* m, int32_t precision, eg_lo** out) {
   cudaMemcpy(perm.data(), m->perm, sizeof(int32_t) * perm.size(), cudaMemcpyDeviceToHost);
   for (int f = 0; f < m->F; ++f)
     for (int s = 0; s < m->S; ++s) spos[(size_t)f * m->Np + perm[(size_t)f * m->S + s]] = s;
+  lo->face_nodes = 0;
+  for (int j = 0; j < m->Np; ++j) {
+    bool on = false;
+    for (int f = 0; f < m->F; ++f) on = on || spos[(size_t)f * m->Np + j] >= 0;
+    lo->face_nodes += on ? 1 : 0;
+  }
   e = cudaMemcpy(lo->spos, spos.data(), sizeof(int32_t) * spos.size(), cudaMemcpyHostToDevice);
   // coupling block (slot * 2 + side) of every element face, -1 on boundaries
   if (e == cudaSuccess) {
@@ -983,7 +989,7 @@ static void ls_free(eg_ls* ls) {
   if (!ls) return;
   eg_gmres_release(ls);
   void* bufs[] = {ls->V, ls->w, ls->z, ls->xT, ls->bT, ls->part, ls->h, ls->y, ls->xd, ls->bd,
-                  ls->dH, ls->dflags, ls->dscal, ls->cfs, ls->dargs};
+                  ls->dH, ls->dflags, ls->dscal, ls->cfs, ls->dargs, ls->G, ls->tpart};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (ls->hh) cudaFreeHost(ls->hh);
@@ -1009,11 +1015,22 @@ extern "C" int eg_ls_create(eg_lo* lo, eg_pc* pc, int32_t restart, eg_ls** out) 
   ls->nblk = EG_GMRES_STREAM_BLOCKS;
   const int64_t N = lo->mesh->ndof;
   const size_t es = lo->prec == EG_F64 ? 8 : 4;
-  cudaError_t e = cudaMalloc(&ls->V, es * (size_t)(restart + 1) * N);
+  cudaError_t e = cudaMalloc(&ls->V, es * eg_basis_values(restart, N));
   if (e == cudaSuccess) e = cudaMalloc(&ls->w, es * N);
   if (e == cudaSuccess) e = cudaMalloc(&ls->z, es * N);
-  if (e == cudaSuccess && lo->mesh->I)
-    e = cudaMalloc(&ls->cfs, es * (size_t)lo->mesh->I * 2 * lo->nb);
+  if (e == cudaSuccess && lo->mesh->I) {
+    const size_t ct = eg_face_tag_bytes(lo->mesh->I, lo->nb, es), pt = eg_part_tag_bytes(es);
+    e = cudaMalloc(&ls->cfs, ct);
+    if (e == cudaSuccess) e = cudaMemset(ls->cfs, 0, ct);
+    if (e == cudaSuccess) e = cudaMalloc(&ls->tpart, pt);
+    if (e == cudaSuccess) e = cudaMemset(ls->tpart, 0, pt);
+  }
+  // without memory for the pushed operators the solver keeps to the stream path
+  if (e == cudaSuccess && lo->mesh->I && !lo->mesh->sparse_face &&
+      cudaMalloc(&ls->G, eg_push_operator_bytes(lo->mesh->E, lo->n, lo->mesh->F, lo->nb, es)) != cudaSuccess) {
+    ls->G = nullptr;
+    cudaGetLastError();
+  }
   if (e == cudaSuccess) e = cudaMalloc(&ls->xT, es * N);
   if (e == cudaSuccess) e = cudaMalloc(&ls->bT, es * N);
   if (e == cudaSuccess) e = cudaMalloc(&ls->part, es * eg_gmres_partials(restart));

@@ -98,10 +98,13 @@ extern "C" int eg_estimate_mem(const eg_mem_query* qy, eg_mem_estimate* out) {
     // block-Jacobi inverses (eg_pc_create)
     pc.add(es * E * n * n);
     // GMRES(m) (eg_ls_create)
-    kry.add(es * (m + 1) * N);                  // Krylov basis
+    kry.add(es * eg_basis_values((int)m, (int64_t)N));  // Krylov basis
     kry.add(es * N);                            // w
     kry.add(es * N);                            // z
-    kry.add(es * I * 2 * nb);                   // pushed coupling products
+    kry.add(eg_face_tag_bytes(I, (int)nb, es));  // pushed coupling products
+    kry.add(eg_part_tag_bytes(es));             // their partial sums
+    if (!qy->face_diagonal)                     // pushed operators
+      kry.add(eg_push_operator_bytes(E, n, F, (int)nb, es));
     kry.add(es * N);                            // x
     kry.add(es * N);                            // b
     kry.add(es * eg_gmres_partials((int)m));     // partial sums

@@ -369,6 +369,7 @@ IterOut newton_graph_iteration(eg_mesh* m, eg_newton_ws* w, double tau_l) {
     return r;
   }
   m->launches += w->nJ + w->nP;
+  ls->trans = 0;
   r.st = eg_gmres_coop(ls);
   if (r.st != EG_OK) return r;
   ce = cudaEventRecord(w->ev[3], s);
@@ -402,6 +403,13 @@ IterOut newton_graph_iteration(eg_mesh* m, eg_newton_ws* w, double tau_l) {
     cudaStreamSynchronize(s);
     eg_set_error("zero pivot in block LU");
     r.st = EG_ERR_LU_PIVOT;
+    r.updated = false;
+    return r;
+  }
+  if (!flags[F_DONE]) {
+    cudaMemcpyAsync(w->qd, w->qsave, 8 * m->ndof, cudaMemcpyDeviceToDevice, s);
+    cudaStreamSynchronize(s);
+    r.st = eg_gmres_gave_up(ls);
     r.updated = false;
     return r;
   }
