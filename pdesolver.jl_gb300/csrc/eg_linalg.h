@@ -137,6 +137,8 @@ bool eg_coop_usable(const eg_ls* ls);
 
 // kernels shared across translation units
 int eg_jacobian_launch(eg_lo* lo, const double* q);
+// X_e = A_e^-1 for the E column-major n x n blocks (eg_block_inverse.cu)
+int eg_block_inverse(eg_mesh* m, int prec, const void* A, void* X, int n);
 // y = J x in the operator precision (device pointers of that precision);
 // with `done` non-null the launch does nothing while *done != 0
 int eg_lo_apply_T(eg_lo* lo, const void* x, void* y, const int* done = nullptr);

@@ -65,81 +65,6 @@ __global__ void k_cpl_apply(DevMesh md, const T* __restrict__ cpl, const int* __
   }
 }
 
-// ---------------------------------------------------------------- block-Jacobi
-// In-place Gauss-Jordan inversion with partial pivoting of one element block
-// per CTA (column-major n x n in shared memory).  Rows are swapped during the
-// elimination; the inverse's columns are swapped back at the end.
-template <typename T>
-__global__ void k_block_inverse(const T* __restrict__ blocks, T* __restrict__ inv, int n,
-                                unsigned int* __restrict__ status) {
-  extern __shared__ unsigned char smraw[];
-  T* A = reinterpret_cast<T*>(smraw);                       // A[c*n + r]
-  int* piv = reinterpret_cast<int*>(A + (size_t)n * n);
-  __shared__ int s_p;
-  __shared__ T s_d;
-  __shared__ int s_bad;
-  const int e = blockIdx.x;
-  const T* src = blocks + (size_t)e * n * n;
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) A[t] = src[t];
-  if (threadIdx.x == 0) s_bad = 0;
-  __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    if (threadIdx.x == 0) {
-      int p = k;
-      T best = fabs(A[(size_t)k * n + k]);
-      for (int i = k + 1; i < n; ++i) {
-        const T v = fabs(A[(size_t)k * n + i]);
-        if (v > best) { best = v; p = i; }
-      }
-      s_p = p;
-      piv[k] = p;
-      if (!(best > T(0))) s_bad = 1;
-    }
-    __syncthreads();
-    const int p = s_p;
-    if (p != k)
-      for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        const T t0 = A[(size_t)c * n + k];
-        A[(size_t)c * n + k] = A[(size_t)c * n + p];
-        A[(size_t)c * n + p] = t0;
-      }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const T piv_v = A[(size_t)k * n + k];
-      s_d = s_bad ? T(0) : T(1) / piv_v;
-      A[(size_t)k * n + k] = T(1);
-    }
-    __syncthreads();
-    const T d = s_d;
-    for (int c = threadIdx.x; c < n; c += blockDim.x) A[(size_t)c * n + k] *= d;  // row k
-    __syncthreads();
-    // eliminate column k from the other rows: A[i][c] -= A[i][k] * A[k][c]
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      const int c = t / n, i = t - c * n;
-      if (i == k || c == k) continue;
-      A[t] -= A[(size_t)k * n + i] * A[(size_t)c * n + k];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-      if (i != k) A[(size_t)k * n + i] = -A[(size_t)k * n + i] * d;
-    __syncthreads();
-  }
-  // undo the row interchanges as column interchanges, last first
-  for (int k = n - 1; k >= 0; --k) {
-    const int p = piv[k];
-    if (p != k)
-      for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        const T t0 = A[(size_t)k * n + r];
-        A[(size_t)k * n + r] = A[(size_t)p * n + r];
-        A[(size_t)p * n + r] = t0;
-      }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && s_bad) atomicOr(status, EG_DEV_LU_PIVOT);
-  T* dst = inv + (size_t)e * n * n;
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) dst[t] = A[t];
-}
-
 // y_e = inv_e x_e (batched dense matrix-vector product, thread per row)
 template <int NB, typename T>
 __global__ void k_block_apply(const T* __restrict__ inv, const T* __restrict__ x, T* __restrict__ y,
@@ -460,188 +385,6 @@ void launch_cpl_transpose(eg_lo* lo, const T* v, const T* z, T* w, const int* do
   eg_phase_end(m, EG_PHASE_OTHER, 1);
 }
 
-// Register-tiled Gauss-Jordan inversion for blocks of 33..128 unknowns, one
-// CTA of NW warps per element block.  Thread (lane, warp) keeps rows
-// lane + 32 r (r < MR) and columns warp + NW c (c < MC) in registers.
-// Partial pivoting is implicit: the pivot of column k is the unused row p of
-// largest |A[p][k]| (ties: lowest row), found by one warp with shuffles; row p
-// is scaled in place and eliminated from the others, so no rows move.  Row p
-// is read by every warp from its own lane p % 32 (shuffles), column k goes
-// through a double-buffered shared array, so one barrier per column suffices.
-// With S the in-place result and perm[k] the pivot row of column k,
-// A^-1[r][c] = S[perm[r]][q] where perm[q] = c.
-// register row r (warp-uniform) of a thread's tile, through branches on the
-// uniform index so that only one copy executes (no per-element selects)
-template <typename T, int MR, int MC>
-__device__ __forceinline__ void tile_row_shfl(const T (&a)[MR][MC], int r, int src_lane, T scale,
-                                              T (&out)[MC]) {
-#pragma unroll
-  for (int rr = 0; rr < MR; ++rr)
-    if (rr == r) {
-#pragma unroll
-      for (int c = 0; c < MC; ++c) out[c] = __shfl_sync(0xffffffffu, a[rr][c], src_lane) * scale;
-    }
-}
-
-template <typename T, int MR, int MC, int NW>
-__global__ void __launch_bounds__(32 * NW) k_block_inverse_reg(const T* __restrict__ blocks,
-                                                                T* __restrict__ inv, int n,
-                                                                unsigned int* __restrict__ status) {
-  extern __shared__ unsigned char smraw[];
-  T* S = reinterpret_cast<T*>(smraw);                      // [n][n] column-major, at the end
-  T* colk = S + (size_t)n * n;                             // [2][32 MR] column k
-  int* sp = reinterpret_cast<int*>(colk + 2 * 32 * MR);    // [2] pivot row
-  int* perm = sp + 2;                                      // [n]
-  int* iperm = perm + n;                                   // [n]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const T* src = blocks + (size_t)blockIdx.x * n * n;
-  T a[MR][MC];
-  unsigned used = 0;  // bit r: row lane + 32 r is a pivot row already (or beyond n)
-#pragma unroll
-  for (int r = 0; r < MR; ++r) {
-    const int i = lane + 32 * r;
-    if (i >= n) used |= 1u << r;
-#pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      const int col = warp + NW * c;
-      a[r][c] = (i < n && col < n) ? src[(size_t)col * n + i] : T(0);
-    }
-  }
-  bool bad = false;
-  for (int k = 0; k < n; ++k) {
-    const int buf = k & 1;
-    T* ck = colk + buf * 32 * MR;
-    const bool kwarp = warp == (k % NW);  // this warp holds column k, as its column kc
-    const int kc = k / NW;
-    if (kwarp) {
-      T best = T(-1);
-      int bi = n;
-#pragma unroll
-      for (int c = 0; c < MC; ++c)
-        if (c == kc) {
-#pragma unroll
-          for (int r = 0; r < MR; ++r) {
-            const T v = a[r][c];
-            ck[lane + 32 * r] = v;
-            // NaN ranks above every number, so some unused row (there are
-            // n - k) is always chosen and the pivot check below flags it
-            const T av = isnan(v) ? T(INFINITY) : fabs(v);
-            if (!((used >> r) & 1u) && av > best) {
-              best = av;
-              bi = lane + 32 * r;
-            }
-          }
-        }
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const T ob = __shfl_xor_sync(0xffffffffu, best, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        if (ob > best || (ob == best && oi < bi)) {
-          best = ob;
-          bi = oi;
-        }
-      }
-      if (lane == 0) sp[buf] = bi;
-    }
-    __syncthreads();
-    const int p = sp[buf];
-    const T pv = ck[p];
-    bad = bad || !(fabs(pv) > T(0));
-    const T d = bad ? T(0) : T(1) / pv;
-    T rc[MC];  // scaled pivot row, this thread's columns
-    tile_row_shfl<T, MR, MC>(a, p >> 5, p & 31, d, rc);
-    // rows: r_i -= f_i r_p (every column; column k is set below)
-#pragma unroll
-    for (int r = 0; r < MR; ++r) {
-      const T f = ck[lane + 32 * r];
-#pragma unroll
-      for (int c = 0; c < MC; ++c) a[r][c] = fma(-f, rc[c], a[r][c]);
-    }
-    // the pivot row becomes the scaled row, column k becomes -f d (d in the
-    // pivot row): the in-place inverse's new column
-    if (lane == (p & 31)) {
-#pragma unroll
-      for (int r = 0; r < MR; ++r)
-        if (r == (p >> 5)) {
-#pragma unroll
-          for (int c = 0; c < MC; ++c) a[r][c] = rc[c];
-          used |= 1u << r;
-        }
-    }
-    if (kwarp) {
-#pragma unroll
-      for (int c = 0; c < MC; ++c)
-        if (c == kc) {
-#pragma unroll
-          for (int r = 0; r < MR; ++r)
-            a[r][c] = (lane + 32 * r == p) ? d : -ck[lane + 32 * r] * d;
-        }
-    }
-    if (threadIdx.x == 0) perm[k] = p;
-  }
-  // gather through shared memory into column-major A^-1
-#pragma unroll
-  for (int r = 0; r < MR; ++r)
-#pragma unroll
-    for (int c = 0; c < MC; ++c) {
-      const int i = lane + 32 * r, col = warp + NW * c;
-      if (i < n && col < n) S[(size_t)col * n + i] = a[r][c];
-    }
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) iperm[perm[k]] = k;
-  __syncthreads();
-  T* dst = inv + (size_t)blockIdx.x * n * n;
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-    const int c = t / n, r = t - c * n;
-    dst[t] = S[(size_t)iperm[c] * n + perm[r]];
-  }
-  if (bad && threadIdx.x == 0) atomicOr(status, EG_DEV_LU_PIVOT);
-}
-
-// dynamic shared memory of k_block_inverse_reg
-template <typename T, int MR>
-size_t block_inverse_reg_smem(int n) {
-  return sizeof(T) * ((size_t)n * n + 2 * 32 * MR) + sizeof(int) * (2 + 2 * (size_t)n);
-}
-
-template <typename T>
-int pccalc_T(eg_pc* pc) {
-  eg_lo* lo = pc->lo;
-  eg_mesh* m = lo->mesh;
-  const int n = lo->n;
-  eg_phase_begin(m, EG_PHASE_OTHER);
-  const T* A = (const T*)lo->diag;
-  T* X = (T*)pc->inv;
-  // MC x NW columns cover the block: 8 warps of 8 or 12 columns up to 96
-  // unknowns; up to 128, 16 warps of 8 columns in FP32 (4 x 8 values and 64
-  // registers per thread, two blocks per SM: 18 % faster than 8 warps of 16
-  // columns on 115-unknown blocks) and 8 warps of 16 columns in FP64 (the
-  // 16-warp tile measured 0.7 % slower there)
-#define EG_INV_REG(MR, MC, NW)                                                                  \
-  {                                                                                           \
-    const size_t smem = block_inverse_reg_smem<T, MR>(n);                                     \
-    cudaFuncSetAttribute(k_block_inverse_reg<T, MR, MC, NW>,                                  \
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);            \
-    k_block_inverse_reg<T, MR, MC, NW><<<m->E, 32 * NW, smem, m->stream>>>(A, X, n, m->status); \
-  }
-  if (n <= 32) {
-    const size_t smem = sizeof(T) * (size_t)n * n + sizeof(int) * n;
-    cudaFuncSetAttribute(k_block_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    k_block_inverse<T><<<m->E, 256, smem, m->stream>>>(A, X, n, m->status);
-  } else if (n <= 64) {
-    EG_INV_REG(2, 8, 8)
-  } else if (n <= 96) {
-    EG_INV_REG(3, 12, 8)
-  } else if (sizeof(T) == 4) {
-    EG_INV_REG(4, 8, 16)
-  } else {
-    EG_INV_REG(4, 16, 8)
-  }
-#undef EG_INV_REG
-  eg_phase_end(m, EG_PHASE_OTHER, 1);
-  return EG_OK;
-}
-
 }  // namespace
 
 size_t eg_lo_coupling_size(const eg_lo* lo) {
@@ -948,13 +691,16 @@ extern "C" int eg_pc_calc(eg_pc* pc) {
     eg_set_error("eg_pc_calc: operator not computed");
     return EG_ERR_INVALID;
   }
+  eg_mesh* m = pc->lo->mesh;
   const int n = pc->lo->n;
   const size_t smem = (pc->lo->prec == EG_F64 ? 8 : 4) * ((size_t)n * n + 256) + sizeof(int) * (2 + 2 * (size_t)n);
   if (n > 128 || smem > 200 * 1024) {
     eg_set_error("eg_pc_calc: element block of %d unknowns exceeds shared memory", n);
     return EG_ERR_UNSUPPORTED;
   }
-  int st = pc->lo->prec == EG_F64 ? pccalc_T<double>(pc) : pccalc_T<float>(pc);
+  eg_phase_begin(m, EG_PHASE_OTHER);
+  const int st = eg_block_inverse(m, pc->lo->prec, pc->lo->diag, pc->inv, n);
+  eg_phase_end(m, EG_PHASE_OTHER, 1);
   if (st != EG_OK) return st;
   EG_CUDA(cudaGetLastError());
   pc->valid = true;
