@@ -111,8 +111,8 @@ void eg_rk4_ws_free(eg_mesh* m);
 // stream belongs to it; EG_ERR_INVALID (with a message naming `who`) otherwise
 int eg_check_device(const eg_mesh* m, const char* who);
 // The RK4 step loop of eg_rk4 (reference rk4.jl:201-330) on the device
-// buffers buf[6][ndof] = x_old, k1, k2, k3, res, q, with q = x_old = the
-// start state already in place and the status word cleared.  use_graphs:
+// buffers buf[6][ndof] (x first, q last), with x = the start state already in
+// place and the status word cleared; the result is in q.  use_graphs:
 // replay captured CUDA graphs of the step (the mesh keeps them) where the
 // stream can be captured.  On return the stream has no work of the loop left
 // when the status is not EG_OK.
@@ -135,8 +135,3 @@ int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* s
 int eg_check_status(eg_mesh* m);
 // phase timers enabled (they take CUDA events from a growing pool)
 bool eg_timing_on(const eg_mesh* m);
-// the RK4 stage kernels of eg_rk4 on m->stream (eg_solvers.cu)
-void eg_launch_rk4_stage(eg_mesh* m, const double* res, const double* xold, double c, double* ks,
-                         double* q);
-void eg_launch_rk4_final(eg_mesh* m, const double* k1, const double* k2, const double* k3,
-                         const double* res, double h, double* xold, double* q);

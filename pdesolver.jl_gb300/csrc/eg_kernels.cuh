@@ -84,7 +84,49 @@ __device__ __forceinline__ void face_lift_smem(const DevMesh& md, const double* 
   }
 }
 
+// What an element kernel does with its residual entries: write them (rk 0),
+// or finish a stage of the classical RK4 step in place of separate passes over
+// the state (reference rk4.jl:201-330 with pde_post_func: k_s = M^-1 R).  The
+// stage's input and output vectors differ, since other elements' face fluxes
+// of the stage may still be read from the input.
+//   1: acc = k, out = x + c k      2: acc += 2 k, out = x + c k
+//   3: out = x + c (acc + k), c = h/6 (out may be x)
+struct Epilogue {
+  int rk;
+  double c;
+  const double* Minv;
+  const double* x;
+  double* acc;
+  double* out;
+};
+// entries [0, n) of the CTA's residual block sres, first entry i0 of the vector
+template <int NV>
+__device__ __forceinline__ void write_residual(const Epilogue& ep, const double* sres, size_t i0, int n) {
+  if (ep.rk == 0) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) ep.out[i0 + t] = sres[t];
+    return;
+  }
+  const double* Mi = ep.Minv + i0 / NV;
+  for (int t = threadIdx.x; t < n; t += blockDim.x) {
+    const double k = Mi[t / NV] * sres[t];
+    const size_t i = i0 + t;
+    if (ep.rk == 3) {
+      ep.out[i] = ep.x[i] + ep.c * (ep.acc[i] + k);
+    } else {
+      ep.acc[i] = ep.rk == 1 ? k : ep.acc[i] + 2 * k;
+      ep.out[i] = ep.x[i] + ep.c * k;
+    }
+  }
+}
+
 DevMesh dev_mesh(const eg_mesh* m);
 int eg_launch_residual(eg_mesh* m, const double* q, double* res);
-int eg_launch_split_element(eg_mesh* m, const double* q, double* res, int epb);
+// face fluxes, then the element kernel with its epilogue
+int eg_launch_stage(eg_mesh* m, const double* q, const Epilogue& ep);
+// the weak form of a small mesh in one launch (eg_small.cu)
+bool eg_small_usable(const eg_mesh* m, const double* q, const Epilogue& ep);
+int eg_launch_small(eg_mesh* m, const double* q, const Epilogue& ep);
+int eg_launch_split_element(eg_mesh* m, const double* q, const Epilogue& ep, int epb);
+// elements per CTA of the element kernel: the mesh's setting, else the built-in choice
+int eg_elements_per_cta(const eg_mesh* m);
 int eg_launch_norm(eg_mesh* m, const double* r, int strongres, double* out_dev);

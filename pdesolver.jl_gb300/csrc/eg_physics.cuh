@@ -358,98 +358,93 @@ __device__ __forceinline__ IRAvg<DIM, T> ir_average(const Gas& g, const T* qL, c
   return r;
 }
 
+// 1/x for x in the normal range: the hardware's approximation (about 2^-20)
+// and one Householder step of third order, r (1 + e + e^2) with e = 1 - x r,
+// so 3 FP64 instructions instead of a division's 9 (FP64 is the scarce pipe)
+__device__ __forceinline__ double fast_rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // Per-node quantities of the Ismail-Roe averages: z1 = sqrt(rho/p),
-// zp = sqrt(rho p), their logarithms and the velocity.  Computed once per node
-// so a pair of nodes needs no square root and no logarithm.
+// zp = sqrt(rho p), their logarithms and z1 times the velocity.  Computed once
+// per node so a pair of nodes needs no square root and no logarithm.
 template <int DIM>
 struct IRNode {
-  double z1, zp, lz1, lzp, u, v, w;
+  double z1, zp, lz1, lzp, zu, zv, zw;
 };
 
 template <int DIM, bool LOGS = true>
 __device__ __forceinline__ IRNode<DIM> ir_node(const Gas& g, const double* q) {
   IRNode<DIM> r;
   const double p = pressure<DIM>(g, q);
-  // t = (rho p)^-1/2: sqrt(rho/p) = rho t, sqrt(rho p) = rho p t, 1/rho = p t^2
+  // t = (rho p)^-1/2: sqrt(rho/p) = rho t, sqrt(rho p) = rho p t, z1/rho = t
   const double t = rsqrt_(q[0] * p);
-  const double rinv = p * t * t;
   r.z1 = q[0] * t;
-  r.zp = q[0] * p * t;
+  r.zp = r.z1 * p;
   if (LOGS) {
     r.lz1 = log(r.z1);
     r.lzp = log(r.zp);
   } else {
     r.lz1 = r.lzp = 0.0;
   }
-  r.u = q[1] * rinv;
-  r.v = q[2] * rinv;
-  r.w = (DIM == 3) ? q[3] * rinv : 0.0;
+  r.zu = q[1] * t;
+  r.zv = q[2] * t;
+  r.zw = (DIM == 3) ? q[3] * t : 0.0;
   return r;
 }
 
-// Logarithmic means for the Ismail-Roe average from precomputed logarithms.
-// The reference's logavg (bc_solvers.jl:942-956) is (aL + aR) / (2 F) with
-// u = f^2, f = (aL - aR)/(aL + aR), and F = 1 + u/3 + u^2/5 + u^3/7 + u^4/9
-// for u < 1e-3, else F = ln(aL/aR) / (2 f).  The average needs the log mean of
-// sqrt(rho p) (L_p), its reciprocal, and the reciprocal of the log mean of
-// sqrt(rho/p) (1/L_1); all three follow from 1/(aL + aR) and F:
-//   L = s/(2F) = (s/2) G(u),  1/L = 2 F / s,
-// with G = 1/F as its series 1 - u/3 - 4u^2/45 - 44u^3/945 - 428u^4/14175
-// (|G F - 1| < 5e-16 for u < 1e-3), and in the logarithmic branch
-//   1/L = (lL - lR)/d,  L = d^2 x and 1/L = (lL - lR)^2 x with x = 1/(d (lL - lR)).
-// A pair costs one division on the series branch: x = 1/(s_1 s_p) gives
-// 1/s_1 = s_p x and 1/s_p = s_1 x.
-__device__ __forceinline__ double logmean_F(double u) {
-  return 1.0 + u * (1.0 / 3.0 + u * (1.0 / 5.0 + u * (1.0 / 7.0 + u * (1.0 / 9.0))));
-}
-__device__ __forceinline__ double logmean_G(double u) {
-  return 1.0 - u * (1.0 / 3.0 + u * (4.0 / 45.0 + u * (44.0 / 945.0 + u * (428.0 / 14175.0))));
-}
-
-// Ismail-Roe averages of two nodes from their per-node quantities.  PRE: the
-// nodes carry their logarithms (computed once per node, for the pairs of an
-// element); otherwise the logarithm of the ratio is taken on the log-mean
-// branch only (a face node pairs each state once).
+// Ismail-Roe averages of two nodes from their per-node quantities.  The
+// reference's logavg (bc_solvers.jl:942-956) is (aL + aR) / (2 F) with u = f^2,
+// f = (aL - aR)/(aL + aR), and F = 1 + u/3 + u^2/5 + u^3/7 + u^4/9 for u < 1e-3,
+// else F = ln(aL/aR) / (2 f).  With s1, sp the sums of z1 and zp, F1, Fp their
+// F and 1/Lp = 2 Fp / sp, 1/L1 = 2 F1 / s1, the averages are
+//   rho = s1 Lp / 2 = s1 sp / (4 Fp),  p1 = sp / s1,
+//   h = gamma/(gamma - 1) p2 / rho + |u|^2/2,
+//   p2 = (gamma + 1)/(2 gamma) Lp / L1 + (gamma - 1)/(2 gamma) p1,
+// and every factor sp cancels from p2 / rho:
+//   h = s1^-2 (2 (gamma + 1)/(gamma - 1) F1 + 2 Fp) + |u|^2/2.
+// 1/Fp is its series 1 - u/3 - 4u^2/45 - 44u^3/945 - 428u^4/14175 (|G F - 1| <
+// 5e-16 for u < 1e-3).  The branch is taken on the high word of u (u just
+// below 1e-3, where both branches agree to round-off): a compare in the
+// integer pipe.  PRE: the nodes carry their logarithms (computed once per
+// node, for the pairs of an element); otherwise the logarithm of the ratio is
+// taken on that branch only (a face node pairs each state once).
 template <int DIM, bool PRE = true>
 __device__ __forceinline__ IRAvg<DIM, double> ir_average_pre(const Gas& g, const IRNode<DIM>& L,
                                                              const IRNode<DIM>& R) {
-  const double gamma = g.gamma, gamma_1 = g.gamma_1;
+  constexpr int kHi = 0x3f50624d;  // high word of 1e-3
+  const double cA = 2.0 * (g.gamma + 1.0) / g.gamma_1;
   IRAvg<DIM, double> r;
-  // sqrt(rho/p): r1 = 1/(z1L + z1R) is also the weight of the velocity averages;
-  // one division for 1/s1 and 1/sp
   const double s1 = L.z1 + R.z1, d1 = L.z1 - R.z1;
   const double sp = L.zp + R.zp, dp = L.zp - R.zp;
-  const double x1p = 1.0 / (s1 * sp);
-  const double r1 = sp * x1p;
-  double inv_l1;
-  if (d1 * d1 < 1e-3 * (s1 * s1)) {
-    const double f = d1 * r1;
-    inv_l1 = 2.0 * logmean_F(f * f) * r1;
+  const double r1 = fast_rcp(s1);
+  const double f1 = d1 * r1, u1 = f1 * f1;
+  const double fp = dp * fast_rcp(sp), up = fp * fp;
+  double e1, ep, G;  // F1 - 1, Fp - 1, 1 / (4 Fp)
+  if (__double2hiint(u1) < kHi) {
+    e1 = u1 * (1.0 / 3.0 + u1 * (1.0 / 5.0 + u1 * (1.0 / 7.0 + u1 * (1.0 / 9.0))));
   } else {
-    inv_l1 = (PRE ? L.lz1 - R.lz1 : log(L.z1 / R.z1)) / d1;
+    e1 = 0.5 * (PRE ? L.lz1 - R.lz1 : log(L.z1 / R.z1)) / f1 - 1.0;
   }
-  // sqrt(rho p)
-  double lp, inv_lp;
-  if (dp * dp < 1e-3 * (sp * sp)) {
-    const double rp = s1 * x1p;
-    const double f = dp * rp, u = f * f;
-    lp = 0.5 * sp * logmean_G(u);
-    inv_lp = 2.0 * logmean_F(u) * rp;
+  if (__double2hiint(up) < kHi) {
+    ep = up * (1.0 / 3.0 + up * (1.0 / 5.0 + up * (1.0 / 7.0 + up * (1.0 / 9.0))));
+    G = 0.25 - up * (0.25 / 3.0 + up * (1.0 / 45.0 + up * (11.0 / 945.0 + up * (107.0 / 14175.0))));
   } else {
-    const double dl = PRE ? L.lzp - R.lzp : log(L.zp / R.zp);
-    const double x = 1.0 / (dp * dl);
-    lp = dp * dp * x;
-    inv_lp = dl * dl * x;
+    const double lr = PRE ? L.lzp - R.lzp : log(L.zp / R.zp);
+    ep = 0.5 * lr / fp - 1.0;
+    G = 0.5 * fp / lr;
   }
-  r.rho_hat = 0.5 * s1 * lp;
-  r.u_hat = (L.z1 * L.u + R.z1 * R.u) * r1;
-  r.v_hat = (L.z1 * L.v + R.z1 * R.v) * r1;
-  r.w_hat = (DIM == 3) ? (L.z1 * L.w + R.z1 * R.w) * r1 : 0.0;
+  r.rho_hat = (s1 * sp) * G;
+  r.u_hat = (L.zu + R.zu) * r1;
+  r.v_hat = (L.zv + R.zv) * r1;
+  r.w_hat = (DIM == 3) ? (L.zw + R.zw) * r1 : 0.0;
   r.p1_hat = sp * r1;
-  const double p2_hat = ((gamma + 1) / (2 * gamma)) * lp * inv_l1 + (gamma_1 / (2 * gamma)) * r.p1_hat;
-  // h = gamma p2 / (rho_hat (gamma - 1)) + |u|^2/2, 1/rho_hat = 2 r1 / L_p
-  r.h_hat = (gamma / gamma_1) * p2_hat * (2.0 * r1 * inv_lp) +
-            0.5 * (r.u_hat * r.u_hat + r.v_hat * r.v_hat + r.w_hat * r.w_hat);
+  double ke = r.u_hat * r.u_hat + r.v_hat * r.v_hat;
+  if (DIM == 3) ke = fma(r.w_hat, r.w_hat, ke);
+  r.h_hat = fma(0.5, ke, (r1 * r1) * fma(2.0, ep, fma(cA, e1, cA + 2.0)));
   return r;
 }
 

@@ -47,14 +47,26 @@ __global__ void k_face_flux(DevMesh md, const double* __restrict__ q, double* __
     const double* cR = md.interp + ((size_t)fR * Nf + iR) * S;
     const int* pL = md.perm + fL * S;
     const int* pR = md.perm + fR * S;
-    for (int s = 0; s < S; ++s) {
-      const double a = cL[s], b = cR[s];
-      const double* xa = q + ((size_t)eL * Np + pL[s]) * NV;
-      const double* xb = q + ((size_t)eR * Np + pR[s]) * NV;
+    if (md.sparse_face) {
+      // face nodes are volume nodes: the interpolation picks one (at 9 nodes a
+      // dense row was 90 of the 240 FP64 instructions of an IR face node)
+      const double* xa = q + ((size_t)eL * Np + pL[i]) * NV;
+      const double* xb = q + ((size_t)eR * Np + pR[iR]) * NV;
 #pragma unroll
       for (int c = 0; c < NV; ++c) {
-        qL[c] = fma(a, xa[c], qL[c]);
-        qR[c] = fma(b, xb[c], qR[c]);
+        qL[c] = xa[c];
+        qR[c] = xb[c];
+      }
+    } else {
+      for (int s = 0; s < S; ++s) {
+        const double a = cL[s], b = cR[s];
+        const double* xa = q + ((size_t)eL * Np + pL[s]) * NV;
+        const double* xb = q + ((size_t)eR * Np + pR[s]) * NV;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) {
+          qL[c] = fma(a, xa[c], qL[c]);
+          qR[c] = fma(b, xb[c], qR[c]);
+        }
       }
     }
     double nrm[DIM];
@@ -75,11 +87,17 @@ __global__ void k_face_flux(DevMesh md, const double* __restrict__ q, double* __
     const int e = md.bfaces[2 * b], f = md.bfaces[2 * b + 1];
     const double* cL = md.interp + ((size_t)f * Nf + i) * S;
     const int* pL = md.perm + f * S;
-    for (int s = 0; s < S; ++s) {
-      const double a = cL[s];
-      const double* xa = q + ((size_t)e * Np + pL[s]) * NV;
+    if (md.sparse_face) {
+      const double* xa = q + ((size_t)e * Np + pL[i]) * NV;
 #pragma unroll
-      for (int c = 0; c < NV; ++c) qL[c] = fma(a, xa[c], qL[c]);
+      for (int c = 0; c < NV; ++c) qL[c] = xa[c];
+    } else {
+      for (int s = 0; s < S; ++s) {
+        const double a = cL[s];
+        const double* xa = q + ((size_t)e * Np + pL[s]) * NV;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) qL[c] = fma(a, xa[c], qL[c]);
+      }
     }
     double nrm[DIM];
 #pragma unroll
@@ -156,7 +174,7 @@ __device__ __forceinline__ void volume_mma(const double* sQ, const double* sF, d
 // the block is then a whole number of warps.
 template <int DIM, bool MMA>
 __global__ void k_element(DevMesh md, const double* __restrict__ q,
-                          const double* __restrict__ fflux, double* __restrict__ res,
+                          const double* __restrict__ fflux, Epilogue ep,
                           unsigned int* __restrict__ status, int epb) {
   constexpr int NV = DIM + 2;
   constexpr int F = DIM + 1;
@@ -218,9 +236,7 @@ __global__ void k_element(DevMesh md, const double* __restrict__ q,
   }
   __syncthreads();
   face_lift_smem<DIM>(md, fflux, sres, sL, sPerm, e0, nloc);
-  // coalesced copy of the CTA's residual block
-  for (int t = threadIdx.x; t < nloc * Np * NV; t += blockDim.x)
-    res[(size_t)e0 * Np * NV + t] = sres[t];
+  write_residual<NV>(ep, sres, (size_t)e0 * Np * NV, nloc * Np * NV);
 }
 
 // sum of r^2 * M^{+-1} per block, then one block reduces the partials in a
@@ -372,39 +388,53 @@ DevMesh dev_mesh(const eg_mesh* m) {
   return d;
 }
 
+// Built-in elements per CTA.  The element kernels are bound by the FP64 pipe,
+// where a warp costs the same with idle lanes, and by the SM that gets the
+// most CTAs: the choice minimises that SM's CTAs (152 SMs) times the warps of a
+// CTA plus the staging of the operator tables (1100 values cost about a warp's
+// work), within 256 threads; of equal choices the largest.  Measured, 256 / Np
+// elements -> this choice: 8,192 triangles p=3 59.8 -> 57.6 us (18 elements),
+// 82,944-tet split form p=2 unchanged (11), 2,058 tets p=2 split form 164 ->
+// 132 us (8), 7,986 tets p=1 split form 75 -> 64 us (5), 2,058 tets p=3 234 ->
+// 192 us (4).
+static int default_epb(const eg_mesh* m) {
+  constexpr int kSM = 152;
+  const int most = m->Np >= 256 ? 1 : 256 / m->Np;
+  const double staging = m->dim * m->Np * m->Np / 1100.0;
+  int best = 1;
+  double cost = -1.0;
+  for (int e = 1; e <= most; ++e) {
+    const int warps = (e * m->Np + 31) / 32, ctas = (m->E + e - 1) / e;
+    const double c = (ctas + kSM - 1) / kSM * (warps + staging);
+    if (cost < 0 || c <= cost) {
+      cost = c;
+      best = e;
+    }
+  }
+  return best;
+}
+
+int eg_elements_per_cta(const eg_mesh* m) { return m->elem_epb > 0 ? m->elem_epb : default_epb(m); }
+
 // Launch shape of the element kernel with `epb` elements per CTA (0: the
-// built-in choice, 256 / Np weak form; the split form as many as fit 160 KB).
-// Weak form: one thread per (element, node), rounded up to whole warps with
-// the tensor-core contraction.  Split form: the pair table of every element
-// in shared memory.
+// built-in choice): one thread per (element, node), rounded up to whole warps
+// with the tensor-core contraction.
 int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* smem) {
   const int nv = m->nv, Np = m->Np;
-  const size_t common = sizeof(double) * ((size_t)m->dim * Np * Np + (size_t)m->F * m->Nf * m->S +
-                                          (size_t)(m->F * m->S + 1) / 2);
-  if (m->params.volume_integral_type == 2) {
-    if (mma) {
-      eg_set_error("launch config: the split form has no tensor-core contraction");
-      return EG_ERR_INVALID;
-    }
-    const int P = Np * (Np - 1) / 2;
-    auto smem_of = [&](int e) {
-      return common + sizeof(double) * ((size_t)e * Np * nv + (size_t)e * P * nv +
-                                        (size_t)e * Np * nv + (size_t)e * Np * 7) +
-             sizeof(short2) * (size_t)P;
-    };
-    if (epb <= 0) {
-      epb = 256 / Np;
-      if (epb < 1) epb = 1;
-      while (epb > 1 && smem_of(epb) > 160 * 1024) --epb;
-    }
-    *smem = smem_of(epb);
+  const bool split = m->params.volume_integral_type == 2;
+  if (split && mma) {
+    eg_set_error("launch config: the split form has no tensor-core contraction");
+    return EG_ERR_INVALID;
+  }
+  if (epb <= 0) epb = default_epb(m);
+  const size_t lift = (size_t)m->F * m->Nf * m->S + (size_t)(m->F * m->S + 1) / 2;
+  if (split) {
+    // pair tables of both orientations, node quantities, residual
+    const size_t nd = 7 + (size_t)m->dim * m->dim;
+    *smem = sizeof(double) * (2 * (size_t)(Np / 2) * m->dim * Np + lift + (size_t)epb * Np * (nd + nv));
     *threads = epb * Np;
   } else {
-    if (epb <= 0) {
-      epb = 256 / Np;
-      if (epb < 1) epb = 1;
-    }
-    *smem = common + sizeof(double) * ((size_t)epb * m->dim * Np * nv + (size_t)epb * Np * nv);
+    *smem = sizeof(double) * ((size_t)m->dim * Np * Np + lift + (size_t)epb * (m->dim + 1) * Np * nv);
     *threads = mma ? (epb * Np + 31) / 32 * 32 : epb * Np;
   }
   if (*threads > 1024 || *smem > 200 * 1024) {
@@ -415,22 +445,10 @@ int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* s
   return EG_OK;
 }
 
-static int effective_epb(const eg_mesh* m) {
-  if (m->elem_epb > 0) return m->elem_epb;
-  int e = 256 / m->Np;
-  if (e < 1) e = 1;
-  if (m->params.volume_integral_type == 2) {
-    int threads;
-    size_t smem;
-    while (e > 1 && (eg_element_shape(m, e, 0, &threads, &smem) != EG_OK || smem > 160 * 1024)) --e;
-  }
-  return e;
-}
-
-int eg_launch_element(eg_mesh* m, const double* q, double* res) {
-  if (m->params.volume_integral_type == 2) return eg_launch_split_element(m, q, res, effective_epb(m));
+static int launch_element(eg_mesh* m, const double* q, const Epilogue& ep) {
+  const int epb = eg_elements_per_cta(m);
+  if (m->params.volume_integral_type == 2) return eg_launch_split_element(m, q, ep, epb);
   DevMesh md = dev_mesh(m);
-  const int epb = effective_epb(m);
   const bool mma = m->vol_mma != 0;
   int threads;
   size_t smem;
@@ -448,23 +466,30 @@ int eg_launch_element(eg_mesh* m, const double* q, double* res) {
   (void)attr_set;
   if (m->dim == 2) {
     if (mma)
-      k_element<2, true><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, res, m->status, epb);
+      k_element<2, true><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
     else
-      k_element<2, false><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, res, m->status, epb);
+      k_element<2, false><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
   } else {
     if (mma)
-      k_element<3, true><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, res, m->status, epb);
+      k_element<3, true><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
     else
-      k_element<3, false><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, res, m->status, epb);
+      k_element<3, false><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
   }
   return EG_OK;
 }
 
-int eg_launch_residual(eg_mesh* m, const double* q, double* res) {
+int eg_launch_element(eg_mesh* m, const double* q, double* res) {
+  return launch_element(m, q, Epilogue{0, 0.0, m->Minv, nullptr, nullptr, res});
+}
+
+int eg_launch_stage(eg_mesh* m, const double* q, const Epilogue& ep) {
+  if (eg_small_usable(m, q, ep)) return eg_launch_small(m, q, ep);
   DevMesh md = dev_mesh(m);
   const int nf_threads = (m->I + m->B) * m->Nf;
   if (nf_threads > 0) {
-    const int nt = 128;
+    // a thread's flux is one long FP64 chain: one-warp CTAs spread few of them
+    // over all SMs
+    const int nt = nf_threads <= 152 * 128 ? 32 : 128;
     eg_phase_begin(m, EG_PHASE_FACE);
     if (m->dim == 2)
       k_face_flux<2><<<(nf_threads + nt - 1) / nt, nt, 0, m->stream>>>(md, q, m->fflux);
@@ -473,9 +498,13 @@ int eg_launch_residual(eg_mesh* m, const double* q, double* res) {
     eg_phase_end(m, EG_PHASE_FACE, 1);
   }
   eg_phase_begin(m, EG_PHASE_ELEMENT);
-  const int st = eg_launch_element(m, q, res);
+  const int st = launch_element(m, q, ep);
   eg_phase_end(m, EG_PHASE_ELEMENT, 1);
   return st;
+}
+
+int eg_launch_residual(eg_mesh* m, const double* q, double* res) {
+  return eg_launch_stage(m, q, Epilogue{0, 0.0, m->Minv, nullptr, nullptr, res});
 }
 
 int eg_launch_norm(eg_mesh* m, const double* r, int strongres, double* out_dev) {

@@ -30,32 +30,6 @@ __global__ void k_axpby64(double a, const double* __restrict__ x, double b, doub
     y[i] = a * x[i] + b * y[i];
 }
 
-// RK4 stage: k_s = M^-1 res (in place into ks), q = x_old + c * k_s
-__global__ void k_rk4_stage(const double* __restrict__ res, const double* __restrict__ Minv,
-                            const double* __restrict__ xold, double c, double* __restrict__ ks,
-                            double* __restrict__ q, int64_t nnode, int nv) {
-  const int64_t N = nnode * nv;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-    const double k = Minv[i / nv] * res[i];
-    ks[i] = k;
-    q[i] = xold[i] + c * k;
-  }
-}
-
-// final RK4 update: x_old += h/6 (k1 + 2 k2 + 2 k3 + k4), q = x_old (k4 = M^-1 res)
-__global__ void k_rk4_final(const double* __restrict__ k1, const double* __restrict__ k2,
-                            const double* __restrict__ k3, const double* __restrict__ res,
-                            const double* __restrict__ Minv, double h, double* __restrict__ xold,
-                            double* __restrict__ q, int64_t nnode, int nv) {
-  const int64_t N = nnode * nv;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-    const double k4 = Minv[i / nv] * res[i];
-    const double x = xold[i] + (h / 6) * (k1[i] + 2 * k2[i] + 2 * k3[i] + k4);
-    xold[i] = x;
-    q[i] = x;
-  }
-}
-
 // pseudo-transient continuation: J(e,(j,a),(j,a)) -= M_j / tau_vec_j with
 // tau_vec = tau_l / (1 + sqrt(jac))  (reference globalization.jl:165-320)
 template <typename T>
@@ -632,7 +606,7 @@ extern "C" int eg_newton_solve(eg_mesh* m, double* q, int32_t mem, const eg_newt
 // the vectors, the step size and the launch configuration they were taken
 // with.
 struct eg_rk4_ws {
-  double* buf = nullptr;  // [6][N]: x_old, k1, k2, k3, res, q
+  double* buf = nullptr;  // [6][N]: x, acc, stage state, unused, unused, q
   bool tried = false;     // capture attempted for `key`
   bool have = false;      // graphs valid for `key`
   struct {
@@ -655,40 +629,31 @@ void rk4_graphs_free(eg_rk4_ws* w) {
   w->have = false;
 }
 
-// stage 1: k1 = M^-1 R(q), q = x_old + h/2 k1, and (with_norm) the norm of
-// k1 weighted by M, sqrt(sum k1^2 M), read back into m->h_red[0]
+// stage 1: acc = k1 = M^-1 R(x), q = x + h/2 k1, and (with_norm) the norm of
+// k1 weighted by M, sqrt(sum k1^2 M), read back into m->h_red[0].  The stages
+// are the epilogue of the element kernel (Epilogue), so a step is 8 launches
+// and no pass over the state of its own.
 int rk4_stage1(eg_mesh* m, double* buf, double h, bool with_norm) {
   const int64_t N = m->ndof;
-  double *xold = buf, *k1 = buf + N, *res = buf + 4 * N, *qd = buf + 5 * N;
-  int st = eg_launch_residual(m, qd, res);
+  double *x = buf, *acc = buf + N, *q = buf + 5 * N;
+  const int st = eg_launch_stage(m, x, Epilogue{1, h / 2, m->Minv, x, acc, q});
   if (st != EG_OK) return st;
-  eg_launch_rk4_stage(m, res, xold, h / 2, k1, qd);
-  m->launches += 1;
   if (with_norm) {
-    eg_launch_norm(m, k1, 0, m->red + 2048);
+    eg_launch_norm(m, acc, 0, m->red + 2048);
     EG_CUDA(cudaMemcpyAsync(m->h_red, m->red + 2048, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   }
   EG_CUDA(cudaGetLastError());
   return EG_OK;
 }
 
-// stages 2, 3, 4 and the update of x_old and q
+// stages 2, 3, 4 and the update of x
 int rk4_rest(eg_mesh* m, double* buf, double h) {
   const int64_t N = m->ndof;
-  double *xold = buf, *k1 = buf + N, *k2 = buf + 2 * N, *k3 = buf + 3 * N, *res = buf + 4 * N,
-         *qd = buf + 5 * N;
-  int st = eg_launch_residual(m, qd, res);
-  if (st == EG_OK) {
-    eg_launch_rk4_stage(m, res, xold, h / 2, k2, qd);
-    st = eg_launch_residual(m, qd, res);
-  }
-  if (st == EG_OK) {
-    eg_launch_rk4_stage(m, res, xold, h, k3, qd);
-    st = eg_launch_residual(m, qd, res);
-  }
+  double *x = buf, *acc = buf + N, *p = buf + 2 * N, *q = buf + 5 * N;
+  int st = eg_launch_stage(m, q, Epilogue{2, h / 2, m->Minv, x, acc, p});
+  if (st == EG_OK) st = eg_launch_stage(m, p, Epilogue{2, h, m->Minv, x, acc, q});
+  if (st == EG_OK) st = eg_launch_stage(m, q, Epilogue{3, h / 6, m->Minv, x, acc, x});
   if (st != EG_OK) return st;
-  eg_launch_rk4_final(m, k1, k2, k3, res, h, xold, qd);
-  m->launches += 3;
   EG_CUDA(cudaGetLastError());
   return EG_OK;
 }
@@ -754,6 +719,7 @@ int eg_rk4_loop(eg_mesh* m, double* buf, double h, double t_max, int itermax, do
   const long t_steps = lround(t_max / h);
   double t = 0.0, last_norm = 0.0;
   int steps = 0, st = EG_OK;
+  bool whole = true;  // the state is x (else q, after a break in stage 1)
   // loop i = 2 .. t_steps+1 of the reference (rk4.jl:201)
   for (long i = 2; i <= t_steps + 1; ++i) {
     t = (i - 2) * h;
@@ -768,6 +734,7 @@ int eg_rk4_loop(eg_mesh* m, double* buf, double h, double t_max, int itermax, do
       ++steps;
       continue;
     }
+    whole = false;
     // stage 1 (with the norm, as pde_post_func with calc_norm=true)
     if (graphs && with_norm) {
       cudaError_t ce = cudaGraphLaunch(w->g_stage1, m->stream);
@@ -803,9 +770,15 @@ int eg_rk4_loop(eg_mesh* m, double* buf, double h, double t_max, int itermax, do
       st = rk4_rest(m, buf, h);
       if (st != EG_OK) break;
     }
+    whole = true;
     ++steps;
   }
   t += h;
+  if (st == EG_OK && whole) {
+    const cudaError_t ce = cudaMemcpyAsync(buf + 5 * m->ndof, buf, 8 * (size_t)m->ndof, cudaMemcpyDeviceToDevice,
+                                           m->stream);
+    if (ce != cudaSuccess) st = eg_cuda_fail(ce, "eg_rk4");
+  }
   // a failed launch leaves earlier work queued: let it finish before the
   // caller reuses or frees the buffers
   if (st != EG_OK) cudaStreamSynchronize(m->stream);
@@ -904,18 +877,4 @@ extern "C" int eg_prolong(eg_mesh* lo, const double* q_lo, eg_mesh* hi, double* 
     EG_CUDA(cudaMemcpyAsync(q_hi, dst, 8 * (size_t)hi->ndof, cudaMemcpyDeviceToHost, hi->stream));
   EG_CUDA(cudaStreamSynchronize(hi->stream));
   return EG_OK;
-}
-
-// RK4 stage launches for other translation units: the kernels, grid and
-// launch counting of eg_rk4
-void eg_launch_rk4_stage(eg_mesh* m, const double* res, const double* xold, double c, double* ks,
-                         double* q) {
-  k_rk4_stage<<<grid64(m->ndof), 256, 0, m->stream>>>(res, m->Minv, xold, c, ks, q,
-                                                      (int64_t)m->E * m->Np, m->nv);
-}
-
-void eg_launch_rk4_final(eg_mesh* m, const double* k1, const double* k2, const double* k3,
-                         const double* res, double h, double* xold, double* q) {
-  k_rk4_final<<<grid64(m->ndof), 256, 0, m->stream>>>(k1, k2, k3, res, m->Minv, h, xold, q,
-                                                      (int64_t)m->E * m->Np, m->nv);
 }

@@ -67,11 +67,13 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
     return EG_ERR_INVALID;
   }
   // candidates: elements per CTA in powers of two and the built-in choice
-  // 256 / Np, times the contraction kind for the weak form
+  // (eg_elements_per_cta), times the contraction kind for the weak form
   std::vector<eg_launch_config> cand;
   const bool weak = m->params.volume_integral_type == 1;
-  int builtin = 256 / m->Np;
-  if (builtin < 1) builtin = 1;
+  const int own_epb = m->elem_epb;
+  m->elem_epb = 0;
+  const int builtin = eg_elements_per_cta(m);
+  m->elem_epb = own_epb;
   std::vector<int> sizes;
   for (int epb = 1; epb <= 128; epb *= 2) {
     if (builtin > epb / 2 && builtin < epb) sizes.push_back(builtin);
@@ -98,8 +100,9 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
   const bool timers = eg_timing_on(m);
   if (timers) eg_set_timing(m, 0);
   double* res = m->res_dev;
-  // face fluxes of q once; every candidate then reads the same m->fflux
-  m->elem_epb = 0;
+  // face fluxes of q once (an explicit configuration keeps to the two
+  // kernels); every candidate then reads the same m->fflux
+  m->elem_epb = builtin;
   m->vol_mma = 0;
   int st = eg_launch_residual(m, q_dev, res);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
