@@ -88,7 +88,8 @@ struct eg_mesh {
   double* res_dev;  // [ndof] staging for host outputs
   unsigned int* status;   // device status word
   double* red;      // reduction scratch
-  unsigned int* h_status; // pinned host mirror
+  unsigned int* h_status; // pinned host mirror, and a word eg_eval_residual's kernels write
+  bool status_clear;      // the device word is known to be zero
   double* h_red;          // pinned host scalar
   cudaStream_t own_stream;  // the library's stream (stream may be a caller's)
   TimerState* timer;        // phase timers (null until enabled)

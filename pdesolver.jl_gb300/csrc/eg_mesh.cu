@@ -338,7 +338,7 @@ extern "C" int eg_mesh_create(const eg_mesh_desc* d, const eg_params* params, eg
     m->stream = m->own_stream;
   }
   if (st == EG_OK) {
-    cudaError_t e1 = cudaMallocHost((void**)&m->h_status, sizeof(unsigned int));
+    cudaError_t e1 = cudaMallocHost((void**)&m->h_status, 2 * sizeof(unsigned int));
     if (e1 == cudaSuccess) e1 = cudaMallocHost((void**)&m->h_red, 64 * sizeof(double));
     if (e1 != cudaSuccess) st = eg_cuda_fail(e1, "cudaMallocHost");
   }

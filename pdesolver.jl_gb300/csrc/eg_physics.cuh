@@ -126,9 +126,35 @@ __host__ __device__ __forceinline__ float val(float a) { return a; }
 using ::sqrt;
 using ::log;
 
-// 1/sqrt(x): CUDA's rsqrt (double) / rsqrtf (float); for a derivative
-// carrier d(x^-1/2) = -x^-3/2 dx / 2
-__device__ __forceinline__ double rsqrt_(double a) { return ::rsqrt(a); }
+// Reciprocal and reciprocal square root in few FP64 instructions (FP64 is the
+// scarce pipe: a warp issues one per 64 cycles): the hardware's approximation
+// (about 2^-20) and one Householder step of third order, 3 instructions
+// instead of a division's 9 and 5 for x^-1/2.  Arguments outside [2^-900,
+// 2^900], zero, infinities and NaN take the plain operation.
+__device__ __forceinline__ bool mid_range(double x) {
+  return (unsigned)((__double2hiint(x) & 0x7fffffff) - 0x07b00000) < 0x70800000u;
+}
+__device__ __forceinline__ double rcp_(double x) {
+  if (!mid_range(x)) return 1.0 / x;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+__device__ __forceinline__ float rcp_(float x) { return 1.0f / x; }
+template <typename R, int N>
+__device__ __forceinline__ Fwd<R, N> rcp_(const Fwd<R, N>& a) {
+  return R(1) / a;
+}
+
+// 1/sqrt(x); for a derivative carrier d(x^-1/2) = -x^-3/2 dx / 2
+__device__ __forceinline__ double rsqrt_(double x) {
+  if (!mid_range(x) || __double2hiint(x) < 0) return ::rsqrt(x);
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
 __device__ __forceinline__ float rsqrt_(float a) { return ::rsqrtf(a); }
 template <typename R, int N>
 __device__ __forceinline__ Fwd<R, N> rsqrt_(const Fwd<R, N>& a) {
@@ -213,7 +239,7 @@ __device__ __forceinline__ void roe_flux(const Gas& g, const T* q, const T* qg, 
   T HR = gamma * qg[NV - 1] * rR - gami * phiR;
   T sqL = q[0] * isL;
   T sqR = qg[0] * isR;
-  T fac = one / (sqL + sqR);
+  T fac = rcp_(sqL + sqR);
   T u = (sqL * uL + sqR * uR) * fac;
   T v = (sqL * vL + sqR * vR) * fac;
   T w = (DIM == 3) ? (sqL * wL + sqR * wR) * fac : T(R(0));
@@ -358,16 +384,6 @@ __device__ __forceinline__ IRAvg<DIM, T> ir_average(const Gas& g, const T* qL, c
   return r;
 }
 
-// 1/x for x in the normal range: the hardware's approximation (about 2^-20)
-// and one Householder step of third order, r (1 + e + e^2) with e = 1 - x r,
-// so 3 FP64 instructions instead of a division's 9 (FP64 is the scarce pipe)
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 // Per-node quantities of the Ismail-Roe averages: z1 = sqrt(rho/p),
 // zp = sqrt(rho p), their logarithms and z1 times the velocity.  Computed once
 // per node so a pair of nodes needs no square root and no logarithm.
@@ -420,9 +436,9 @@ __device__ __forceinline__ IRAvg<DIM, double> ir_average_pre(const Gas& g, const
   IRAvg<DIM, double> r;
   const double s1 = L.z1 + R.z1, d1 = L.z1 - R.z1;
   const double sp = L.zp + R.zp, dp = L.zp - R.zp;
-  const double r1 = fast_rcp(s1);
+  const double r1 = rcp_(s1);
   const double f1 = d1 * r1, u1 = f1 * f1;
-  const double fp = dp * fast_rcp(sp), up = fp * fp;
+  const double fp = dp * rcp_(sp), up = fp * fp;
   double e1, ep, G;  // F1 - 1, Fp - 1, 1 / (4 Fp)
   if (__double2hiint(u1) < kHi) {
     e1 = u1 * (1.0 / 3.0 + u1 * (1.0 / 5.0 + u1 * (1.0 / 7.0 + u1 * (1.0 / 9.0))));

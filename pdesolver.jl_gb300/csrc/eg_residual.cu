@@ -446,6 +446,7 @@ int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* s
 }
 
 static int launch_element(eg_mesh* m, const double* q, const Epilogue& ep) {
+  m->status_clear = false;
   const int epb = eg_elements_per_cta(m);
   if (m->params.volume_integral_type == 2) return eg_launch_split_element(m, q, ep, epb);
   DevMesh md = dev_mesh(m);
@@ -483,6 +484,7 @@ int eg_launch_element(eg_mesh* m, const double* q, double* res) {
 }
 
 int eg_launch_stage(eg_mesh* m, const double* q, const Epilogue& ep) {
+  m->status_clear = false;
   if (eg_small_usable(m, q, ep)) return eg_launch_small(m, q, ep);
   DevMesh md = dev_mesh(m);
   const int nf_threads = (m->I + m->B) * m->Nf;
@@ -553,14 +555,30 @@ extern "C" int eg_eval_residual(eg_mesh* m, const double* q, double* res, double
     qd = m->q_dev;
     rd = m->res_dev;
   }
-  EG_CUDA(cudaMemsetAsync(m->status, 0, sizeof(unsigned int), m->stream));
+  // The kernels report an unphysical state straight into a pinned host word
+  // (h_status[1], which only this call uses; touched only when something is
+  // wrong): no memset and no copy between the caller and a small residual.
+  // This call ends synchronised, so nothing of an earlier one is in flight.
+  // The device word is cleared when other work may have set it, and takes the
+  // flags of an unphysical state, as if the kernels had written it.
+  if (!m->status_clear) EG_CUDA(cudaMemsetAsync(m->status, 0, sizeof(unsigned int), m->stream));
+  unsigned int* const dev_status = m->status;
+  volatile unsigned int* word = m->h_status + 1;
+  *word = 0;
+  m->status = m->h_status + 1;
   int st = eg_launch_residual(m, qd, rd);
+  m->status = dev_status;
+  m->status_clear = true;
   if (st != EG_OK) return st;
   EG_CUDA(cudaGetLastError());
-  EG_CUDA(cudaMemcpyAsync(m->h_status, m->status, sizeof(unsigned int), cudaMemcpyDeviceToHost, m->stream));
   if (mem == EG_MEM_HOST)
     EG_CUDA(cudaMemcpyAsync(res, rd, bytes, cudaMemcpyDeviceToHost, m->stream));
   EG_CUDA(cudaStreamSynchronize(m->stream));
+  *m->h_status = *word;
+  if (*word) {
+    m->status_clear = false;
+    EG_CUDA(cudaMemcpyAsync(m->status, m->h_status, sizeof(unsigned int), cudaMemcpyHostToDevice, m->stream));
+  }
   return eg_check_status(m);
 }
 

@@ -478,6 +478,7 @@ extern "C" int eg_newton_solve(eg_mesh* m, double* q, int32_t mem, const eg_newt
   const int64_t N = m->ndof;
   eg_newton_stats s;
   std::memset(&s, 0, sizeof(s));
+  m->status_clear = false;
   eg_newton_ws* w = nullptr;
   int st = newton_ws(m, o->precision, o->gmres_restart > 0 ? o->gmres_restart : 30, &w);
   if (st != EG_OK) return st;
@@ -715,6 +716,7 @@ int eg_rk4_loop(eg_mesh* m, double* buf, double h, double t_max, int itermax, do
   eg_rk4_ws* w = m->rws;
   const bool graphs = use_graphs && w && w->buf == buf && !eg_timing_on(m) && !m->capturing &&
                       rk4_graphs(m, w, h);
+  m->status_clear = false;  // (graph replays)
   const bool with_norm = res_tol > 0;
   const long t_steps = lround(t_max / h);
   double t = 0.0, last_norm = 0.0;
