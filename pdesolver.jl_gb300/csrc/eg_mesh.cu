@@ -125,7 +125,7 @@ static void free_mesh(eg_mesh* m) {
   eg_newton_ws_free(m);
   eg_rk4_ws_free(m);
   if (m->prolong_T) cudaFree(m->prolong_T);
-  void* bufs[] = {m->Q, m->w, m->interp, m->perm, m->nbrperm, m->wface, m->lift, m->liftS,
+  void* bufs[] = {m->Q, m->w, m->interp, m->perm, m->nbrperm, m->wface, m->Qpair, m->liftS,
                   m->nbrinv, m->dxidx,
                   m->jac, m->Minv, m->ifaces, m->nrm_face, m->bfaces, m->bc_of_b,
                   m->coords_bndry, m->nrm_bndry, m->qg_bndry, m->eface, m->fflux,
@@ -276,18 +276,28 @@ extern "C" int eg_mesh_create(const eg_mesh_desc* d, const eg_params* params, eg
       free_mesh(m);
       return EG_ERR_INVALID;
     }
-  // lift[f][j][i] = sum_s [perm[f][s] == j] interp[f][i][s] * wface[i]
-  std::vector<double> lift((size_t)F * Np * Nf, 0.0);
-  for (int f = 0; f < F; ++f)
-    for (int i = 0; i < Nf; ++i)
-      for (int s = 0; s < S; ++s)
-        lift[((size_t)f * Np + d->perm[f * S + s]) * Nf + i] +=
-            d->interp[((size_t)f * Nf + i) * S + s] * d->wface[i];
   std::vector<double> liftS((size_t)F * Nf * S);
   for (int f = 0; f < F; ++f)
     for (int i = 0; i < Nf; ++i)
       for (int s = 0; s < S; ++s)
         liftS[((size_t)f * Nf + i) * S + s] = d->interp[((size_t)f * Nf + i) * S + s] * d->wface[i];
+  // Q entries of the split form's node pairs (j, j + s mod Np), s = 1 .. Np/2,
+  // as 60-bit fixed point relative to 2^Qexp > max |Q| (eg_split.cu)
+  const int H = Np / 2;
+  double qmax = 0.0;
+  for (int k = 0; k < dim * Np * Np; ++k) qmax = std::fmax(qmax, std::fabs(d->Q[k]));
+  m->Qexp = qmax > 0.0 && std::isfinite(qmax) ? std::ilogb(qmax) + 1 : 1;
+  std::vector<int32_t> Qpair((size_t)2 * H * dim * Np * 2);
+  for (int t = 0; t < H * dim * Np; ++t) {
+    const int s = t / (dim * Np), k = (t / Np) % dim, j = t % Np, o = (j + s + 1) % Np;
+    for (int side = 0; side < 2; ++side) {  // Q_k(j, o), Q_k(o, j)
+      const double x = d->Q[((size_t)k * Np + (side ? j : o)) * Np + (side ? o : j)];
+      const long long v = std::isfinite(x) ? std::llrint(std::ldexp(x, 59 - m->Qexp)) : 0;
+      int32_t* q = Qpair.data() + ((size_t)side * H * dim * Np + t) * 2;
+      q[0] = (int32_t)(v >> 30);
+      q[1] = (int32_t)(v & 0x3fffffff);
+    }
+  }
   std::vector<int32_t> nbrinv((size_t)m->norient * Nf);
   for (int o = 0; o < m->norient; ++o)
     for (int i = 0; i < Nf; ++i) nbrinv[(size_t)o * Nf + d->nbrperm[o * Nf + i]] = i;
@@ -312,9 +322,9 @@ extern "C" int eg_mesh_create(const eg_mesh_desc* d, const eg_params* params, eg
   UP(perm, d->perm, (size_t)F * S, "perm");
   UP(nbrperm, d->nbrperm, (size_t)m->norient * Nf, "nbrperm");
   UP(wface, d->wface, (size_t)Nf, "wface");
-  UP(lift, lift.data(), lift.size(), "lift");
   UP(liftS, liftS.data(), liftS.size(), "liftS");
   UP(nbrinv, nbrinv.data(), nbrinv.size(), "nbrinv");
+  UP(Qpair, Qpair.data(), Qpair.size(), "Qpair");
   UP(dxidx, d->dxidx, (size_t)E * Np * dim * dim, "dxidx");
   UP(jac, d->jac, (size_t)E * Np, "jac");
   UP(Minv, minv.data(), minv.size(), "Minv");

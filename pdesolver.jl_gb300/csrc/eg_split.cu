@@ -20,11 +20,21 @@
 // The Q entries of a distance are laid out by j, so the threads read them and
 // the other node's quantities without bank conflicts.
 //
-// Bound: the FP64 pipe.  A pair costs 84 FP64 instructions (the averages from
+// The directions n_jk (18 multiply-adds per pair) are formed in the integer
+// pipe, which has room: metrics and Q entries as 60-bit fixed-point numbers
+// relative to the element's largest metric term and the largest |Q|, in two
+// 30-bit limbs; n_jk = sum of 2 DIM products, high x high and the two cross
+// terms in 64-bit accumulators (the low x low terms are below 2^-57 of full
+// scale), converted to FP64 once.  56 bits doubled the error of the residual
+// against 64-bit arithmetic; with 60 it is that of FP64 directions.  G is linear in n_jk, so
+// the scale is applied to the finished row.
+//
+// Bound: the FP64 pipe.  A pair costs 69 FP64 instructions (the averages from
 // the per-node quantities with two approximate reciprocals, see
 // ir_average_pre); 117 with a division, four threshold tests and separate
 // means, and a table of all pair fluxes in shared memory (17 KB per element,
-// one CTA per SM).  82,944 tets p=2, residual: 6.72 -> 3.92 ms.
+// one CTA per SM).  82,944 tets p=2, residual: 6.72 -> 3.81 ms with n_jk in
+// FP64, 3.42 ms in fixed point.
 #include "eg_internal.h"
 #include "eg_kernels.cuh"
 #include "eg_physics.cuh"
@@ -33,33 +43,53 @@ using eg::Gas;
 
 namespace {
 
+// Fixed point: round(x 2^(59 - ex)), |x| < 2^ex, as high limb (signed, 30
+// bits) and low limb (30 bits).
+struct Limbs {
+  int h, l;
+};
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// smallest e with |x| < 2^e for the largest high word of |x| (normal range; 0
+// and subnormals count as 2^-1022, infinities and NaN as 2^1024)
+__device__ __forceinline__ int exponent_above(int hi) {
+  const int b = (hi >> 20) & 0x7ff;
+  return (b < 1 ? 1 : b) - 1022;
+}
+__device__ __forceinline__ Limbs to_limbs(double x, int ex) {
+  // two exact scalings: 59 - ex may exceed the exponent range of one
+  const int k = 59 - ex, k1 = k / 2;
+  const long long v = __double2ll_rn(x * pow2(k1) * pow2(k - k1));
+  return Limbs{(int)(v >> 30), (int)(v & 0x3fffffff)};
+}
+
 template <int DIM>
 __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
                                 const double* __restrict__ fflux, Epilogue ep,
                                 unsigned int* __restrict__ status, int epb) {
   constexpr int NV = DIM + 2;
   constexpr int F = DIM + 1;
-  constexpr int ND = 7 + DIM * DIM;
+  constexpr int D2 = DIM * DIM;
   extern __shared__ double smem[];
   const int Np = md.Np, Nf = md.Nf, S = md.S;
   const int H = Np / 2;
   const int rows = epb * Np;
-  double* sQa = smem;                         // [H][DIM][Np]: Q_m(j, j + s)
-  double* sQb = sQa + H * DIM * Np;           // [H][DIM][Np]: Q_m(j + s, j)
-  double* sL = sQb + H * DIM * Np;            // [F][Nf][S]
+  Limbs* sQa = reinterpret_cast<Limbs*>(smem);  // [H][DIM][Np]: Q_m(j, j + s)
+  Limbs* sQb = sQa + H * DIM * Np;            // [H][DIM][Np]: Q_m(j + s, j)
+  double* sL = reinterpret_cast<double*>(sQb + H * DIM * Np);  // [F][Nf][S]
   int* sPerm = reinterpret_cast<int*>(sL + F * Nf * S);
-  double* sN = sL + F * Nf * S + (F * S + 1) / 2;  // [ND][rows]: IR quantities, metrics
-  double* sres = sN + (size_t)ND * rows;      // [epb][Np][NV]
-  for (int t = threadIdx.x; t < H * DIM * Np; t += blockDim.x) {
-    const int s = t / (DIM * Np), r = t - s * DIM * Np;
-    const int m = r / Np, j = r - m * Np;
-    int k = j + s + 1;
-    if (k >= Np) k -= Np;
-    sQa[t] = md.Q[((size_t)m * Np + k) * Np + j];  // md.Q[m][k][j] = Q_m(j, k)
-    sQb[t] = md.Q[((size_t)m * Np + j) * Np + k];
+  double* sN = sL + F * Nf * S + (F * S + 1) / 2;  // [7][rows]: IR quantities
+  Limbs* sD = reinterpret_cast<Limbs*>(sN + (size_t)7 * rows);  // [DIM DIM][rows]: metrics
+  double* sres = reinterpret_cast<double*>(sD + (size_t)D2 * rows);  // [epb][Np][NV]
+  int* sMax = reinterpret_cast<int*>(sres + (size_t)rows * NV);  // [epb] largest high word of |dxidx|
+  for (int k = threadIdx.x; k < epb; k += blockDim.x) sMax[k] = 0;
+  const int exQ = md.Qexp;
+  for (int k = threadIdx.x; k < 2 * H * DIM * Np; k += blockDim.x) {
+    const int2 v = md.Qpair[k];
+    sQa[k] = Limbs{v.x, v.y};
   }
   for (int k = threadIdx.x; k < F * Nf * S; k += blockDim.x) sL[k] = md.liftS[k];
   for (int k = threadIdx.x; k < F * S; k += blockDim.x) sPerm[k] = md.perm[k];
+  __syncthreads();  // sMax
   const int e0 = blockIdx.x * epb;
   const int nloc = min(epb, md.E - e0);
   const int t = threadIdx.x;
@@ -67,23 +97,29 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
   const bool active = le < nloc;
   const Gas g{md.gamma, md.gamma_1};
   eg::IRNode<DIM> nd = {};
-  double dx[DIM * DIM];  // [x][xi] of the own node
+  double dxd[D2];
+  Limbs dx[D2];  // metrics [x][xi] of the own node
   double acc[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) acc[c] = 0.0;
 #pragma unroll
-  for (int c = 0; c < DIM * DIM; ++c) dx[c] = 0.0;
+  for (int c = 0; c < D2; ++c) {
+    dxd[c] = 0.0;
+    dx[c] = Limbs{0, 0};
+  }
   if (active) {
     double qj[NV];
     const double* src = q + ((size_t)e0 * Np + t) * NV;
 #pragma unroll
     for (int c = 0; c < NV; ++c) qj[c] = src[c];
-    const double* dxj = md.dxidx + ((size_t)e0 * Np + t) * DIM * DIM;
+    const double* dxj = md.dxidx + ((size_t)e0 * Np + t) * D2;
+    int hi = 0;
 #pragma unroll
-    for (int c = 0; c < DIM * DIM; ++c) {
-      dx[c] = dxj[c];
-      sN[(7 + c) * rows + t] = dx[c];
+    for (int c = 0; c < D2; ++c) {
+      dxd[c] = dxj[c];
+      hi = max(hi, __double2hiint(dxd[c]) & 0x7fffffff);
     }
+    atomicMax(&sMax[le], hi);
     const double pj = eg::pressure<DIM>(g, qj);
     if (!(qj[0] > 0.0)) atomicOr(status, EG_DEV_NEG_DENSITY);
     if (!(pj > 0.0)) atomicOr(status, EG_DEV_NEG_PRESSURE);
@@ -97,6 +133,11 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
     for (int c = 0; c < NV; ++c) sres[(size_t)t * NV + c] = 0.0;
   }
   __syncthreads();
+  const int exD = active ? exponent_above(sMax[le]) : 0;
+  if (active) {
+#pragma unroll
+    for (int c = 0; c < D2; ++c) sD[c * rows + t] = dx[c] = to_limbs(dxd[c], exD);
+  }
   // The logarithms are for pairs whose ratio of z1 or zp exceeds 1.065 (u above
   // 1e-3).  Nodes all within 3 % of the element's first have no such pair
   // (1.03 / 0.97 = 1.062), and the CTA then skips them (two per node were 8 %
@@ -120,18 +161,24 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
     // even Np: distance Np/2 pairs each node with its opposite once
     if (active && (2 * (s + 1) < Np || j < H)) {
       const int o = le * Np + k;
-      const double* qa = sQa + s * DIM * Np + j;
-      const double* qb = sQb + s * DIM * Np + j;
-      double n[DIM];  // 2 S_x[j,k,:]
+      Limbs qa[DIM], qb[DIM];
+#pragma unroll
+      for (int m = 0; m < DIM; ++m) {
+        qa[m] = sQa[(s * DIM + m) * Np + j];
+        qb[m] = sQb[(s * DIM + m) * Np + j];
+      }
+      double n[DIM];  // 2 S_x[j,k,:] times 2^(60 - exD - exQ)
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
-        double v = 0.0;
+        long long hh = 0, x = 0;
 #pragma unroll
         for (int m = 0; m < DIM; ++m) {
-          v = fma(dx[d * DIM + m], qa[m * Np], v);
-          v = fma(-sN[(7 + d * DIM + m) * rows + o], qb[m * Np], v);
+          const Limbs a = dx[d * DIM + m], b = sD[(d * DIM + m) * rows + o];
+          hh += (long long)a.h * qa[m].h - (long long)b.h * qb[m].h;
+          x += (long long)a.h * qa[m].l + (long long)a.l * qa[m].h;
+          x -= (long long)b.h * qb[m].l + (long long)b.l * qb[m].h;
         }
-        n[d] = v;
+        n[d] = (double)((hh << 2) + (x >> 28));
       }
       const eg::IRNode<DIM> no{sN[0 * rows + o], sN[1 * rows + o], sN[2 * rows + o], sN[3 * rows + o],
                                sN[4 * rows + o], sN[5 * rows + o], sN[6 * rows + o]};
@@ -148,8 +195,14 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
     __syncthreads();
   }
   if (active) {
+    // value = n 2^(exD + exQ - 60)
+    const int k = exD + exQ - 60, k1 = k / 2;
+    const double f1 = pow2(k1), f2 = pow2(k - k1);
 #pragma unroll
-    for (int c = 0; c < NV; ++c) sres[(size_t)t * NV + c] += acc[c];
+    for (int c = 0; c < NV; ++c) {
+      double* r = sres + (size_t)t * NV + c;
+      *r = (*r + acc[c]) * f1 * f2;
+    }
   }
   __syncthreads();
   face_lift_smem<DIM>(md, fflux, sres, sL, sPerm, e0, nloc);
