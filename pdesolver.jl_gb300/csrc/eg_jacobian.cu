@@ -169,61 +169,110 @@ __device__ void elem_face_terms(const DevMesh& md, const T* __restrict__ dF, T* 
 }
 
 // Element block: one CTA per element.  Shared: A[k][m][a][b] (flux
-// Jacobians at the nodes), the block blk[col][row] and face tables.  With
-// block_in_global (blocks too large for shared memory, e.g. 225 unknowns of
-// the p=3 diagonal-E tetrahedron) the block is accumulated in place in the
-// output: every entry has one writer per pass, passes are separated by
-// __syncthreads, which orders the CTA's global accesses as well.
+// Jacobians at the nodes), Q, the block blk[col][row], the face operators
+// T[f][i][s][s'] = lift interp and the own-side flux Jacobians D[f][i][a][b] of
+// the element's faces.  A thread owns a row and takes the NV columns of every
+// P-th node, then for each face the NV columns of a stencil node: an entry
+// costs its DIM (Nf) multiply-adds and no index arithmetic.  The face tables
+// are read from memory where they do not fit beside the block
+// (face_tables = 0).  With block_in_global (blocks too large for shared
+// memory) the block is accumulated in place in the output: every entry has
+// one writer per pass, passes are separated by __syncthreads, which orders
+// the CTA's global accesses as well.  With the closed-form flux Jacobians and
+// the dense coupling kernel below, the whole evaluation of 8,192 triangles p=3
+// went from 477 to 362 us in FP64 and from 221 to 87 us in FP32; Omega p=3,
+// whose faces see every node, from 1497 to 973 and 1058 to 212 us.
 template <int DIM, typename T>
-__global__ void k_elem_jac(DevMesh md, const double* __restrict__ q, const T* __restrict__ dF,
-                           T* __restrict__ diag, int block_in_global) {
+__global__ void __launch_bounds__(256) k_elem_jac(DevMesh md, const double* __restrict__ q, const T* __restrict__ dF,
+                                                  T* __restrict__ diag, int block_in_global, int face_tables) {
   constexpr int NV = DIM + 2;
-  using D1 = Fwd<T, NV>;
+  constexpr int F = DIM + 1;
   extern __shared__ unsigned char smraw[];
-  const int Np = md.Np;
+  const int Np = md.Np, Nf = md.Nf, S = md.S;
   const int n = Np * NV;
   const int e = blockIdx.x;
-  T* sA = reinterpret_cast<T*>(smraw);               // [DIM][Np][NV][NV]
-  T* sQ = sA + (size_t)DIM * Np * NV * NV;            // [DIM][Np][Np] = Q
+  T* sA = reinterpret_cast<T*>(smraw);       // [DIM][Np][NV][NV]
+  T* sQ = sA + (size_t)DIM * Np * NV * NV;   // [DIM][Np][Np] = Q
+  T* sT = sQ + (size_t)DIM * Np * Np;        // [F][Nf][S][S]
+  T* sD = sT + (size_t)F * Nf * S * S;       // [F][Nf][NV][NV]
   T* sB = block_in_global ? diag + (size_t)e * n * n  // [n][n] col-major
-                          : sQ + (size_t)DIM * Np * Np;
+                          : sT + (face_tables ? (size_t)F * Nf * (S * S + NV * NV) : 0);
   for (int t = threadIdx.x; t < DIM * Np * Np; t += blockDim.x) sQ[t] = T(md.Q[t]);
+  for (int t = threadIdx.x; face_tables && t < F * Nf * S * S; t += blockDim.x) {
+    const int fi = t / (S * S), ss = t - fi * S * S;
+    sT[t] = T(md.liftS[(size_t)fi * S + ss / S]) * T(md.interp[(size_t)fi * S + ss % S]);
+  }
+  for (int t = threadIdx.x; face_tables && t < F * Nf * NV * NV; t += blockDim.x) {
+    const int f = t / (Nf * NV * NV), r = t - f * Nf * NV * NV;
+    const EFace ef = md.eface[(size_t)e * F + f];
+    const int i = r / (NV * NV), ab = r - i * NV * NV;
+    sD[t] = dF[((size_t)ef.slot * Nf + i) * 2 * NV * NV + (ef.side ? NV * NV : 0) + ab];
+  }
   const Gas g{md.gamma, md.gamma_1};
   // flux Jacobians A_k(q_m) = dF_k/dq at node m, direction dxidx[.][k]
   for (int t = threadIdx.x; t < Np * DIM; t += blockDim.x) {
     const int m = t / DIM, k = t - m * DIM;
     const double* src = q + ((size_t)e * Np + m) * NV;
-    D1 qm[NV], Fk[NV];
+    T qm[NV];
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      qm[c] = D1(T(src[c]));
-      qm[c].d[c] = T(1);
-    }
+    for (int c = 0; c < NV; ++c) qm[c] = T(src[c]);
     const double* dx = md.dxidx + ((size_t)e * Np + m) * DIM * DIM;
     T dir[DIM];
 #pragma unroll
     for (int pp = 0; pp < DIM; ++pp) dir[pp] = T(dx[pp * DIM + k]);
-    eg::euler_flux<DIM>(g, qm, dir, Fk);
-    T* A = sA + (((size_t)k * Np + m) * NV) * NV;
-#pragma unroll
-    for (int a = 0; a < NV; ++a)
-#pragma unroll
-      for (int b = 0; b < NV; ++b) A[a * NV + b] = Fk[a].d[b];
+    eg::euler_flux_jac<DIM>(g, qm, dir, sA + (((size_t)k * Np + m) * NV) * NV);
   }
   __syncthreads();
   // volume: blk[(m,b)][(j,a)] = sum_k Q_k(m, j) A_k(m)[a][b];  Q[k][j][m] = Q_k(m, j)
-  for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-    const int col = t / n, row = t - col * n;
-    const int m = col / NV, b = col - m * NV;
-    const int j = row / NV, a = row - j * NV;
-    T acc = T(0);
+  const int P = n < (int)blockDim.x ? blockDim.x / n : 1;
+  const int part = threadIdx.x / n;
+  for (int r = P > 1 ? threadIdx.x - part * n : threadIdx.x; r < n; r += P > 1 ? n : blockDim.x) {
+    if (P > 1 && part >= P) break;
+    const int j = r / NV, a = r - j * NV;
+    for (int m = P > 1 ? part : 0; m < Np; m += P) {
+      T v[NV];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k)
-      acc += sQ[((size_t)k * Np + j) * Np + m] * sA[(((size_t)k * Np + m) * NV + a) * NV + b];
-    sB[t] = acc;
+      for (int b = 0; b < NV; ++b) v[b] = T(0);
+#pragma unroll
+      for (int k = 0; k < DIM; ++k) {
+        const T w = sQ[((size_t)k * Np + j) * Np + m];
+        const T* A = sA + (((size_t)k * Np + m) * NV + a) * NV;
+#pragma unroll
+        for (int b = 0; b < NV; ++b) v[b] += w * A[b];
+      }
+#pragma unroll
+      for (int b = 0; b < NV; ++b) sB[(size_t)(m * NV + b) * n + r] = v[b];
+    }
   }
   __syncthreads();
-  elem_face_terms<DIM, T>(md, dF, sB, e);
+  // the element's own face terms (LL for elementL / boundary, RR for elementR)
+  for (int f = 0; f < F; ++f) {
+    const EFace ef = md.eface[(size_t)e * F + f];
+    const T sgn = ef.side ? T(1) : T(-1);
+    const int* nb = md.nbrperm + ef.orient * Nf;
+    const int rows = S * NV;
+    const T* Df = face_tables ? sD + (size_t)f * Nf * NV * NV
+                              : dF + (size_t)ef.slot * Nf * 2 * NV * NV + (ef.side ? NV * NV : 0);
+    const int dstep = face_tables ? NV * NV : 2 * NV * NV;
+    for (int t = threadIdx.x; t < rows * S; t += blockDim.x) {
+      const int sp = t / rows, ra = t - sp * rows;  // column stencil node, row (s, a)
+      const int s = ra / NV, a = ra - s * NV;
+      T v[NV];
+#pragma unroll
+      for (int b = 0; b < NV; ++b) v[b] = T(0);
+      for (int i = 0; i < Nf; ++i) {
+        const size_t fi = (size_t)f * Nf + (ef.side ? nb[i] : i);
+        const T w = face_tables ? sT[(fi * S + s) * S + sp] : T(md.liftS[fi * S + s]) * T(md.interp[fi * S + sp]);
+        const T* D = Df + (size_t)i * dstep + a * NV;
+#pragma unroll
+        for (int b = 0; b < NV; ++b) v[b] += w * D[b];
+      }
+      T* dst = sB + (size_t)md.perm[f * S + sp] * NV * n + md.perm[f * S + s] * NV + a;
+#pragma unroll
+      for (int b = 0; b < NV; ++b) dst[(size_t)b * n] += sgn * v[b];
+    }
+    __syncthreads();
+  }
   if (block_in_global) return;
   T* dst = diag + (size_t)e * n * n;
   for (int t = threadIdx.x; t < n * n; t += blockDim.x) dst[t] = sB[t];
@@ -240,7 +289,6 @@ __global__ void __launch_bounds__(128) k_elem_jac_diag(DevMesh md, const double*
                                                        const T* __restrict__ dF, T* __restrict__ diag) {
   constexpr int NV = DIM + 2;
   constexpr int F = DIM + 1;
-  using D1 = Fwd<T, NV>;
   extern __shared__ unsigned char smraw[];
   const int Np = md.Np, Nf = md.Nf, S = md.S;
   const int n = Np * NV;
@@ -252,22 +300,14 @@ __global__ void __launch_bounds__(128) k_elem_jac_diag(DevMesh md, const double*
   for (int t = threadIdx.x; t < Np * DIM; t += blockDim.x) {
     const int m = t / DIM, k = t - m * DIM;
     const double* src = q + ((size_t)e * Np + m) * NV;
-    D1 qm[NV], Fk[NV];
+    T qm[NV];
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      qm[c] = D1(T(src[c]));
-      qm[c].d[c] = T(1);
-    }
+    for (int c = 0; c < NV; ++c) qm[c] = T(src[c]);
     const double* dx = md.dxidx + ((size_t)e * Np + m) * DIM * DIM;
     T dir[DIM];
 #pragma unroll
     for (int pp = 0; pp < DIM; ++pp) dir[pp] = T(dx[pp * DIM + k]);
-    eg::euler_flux<DIM>(g, qm, dir, Fk);
-    T* A = sA + (((size_t)k * Np + m) * NV) * NV;
-#pragma unroll
-    for (int a = 0; a < NV; ++a)
-#pragma unroll
-      for (int b = 0; b < NV; ++b) A[a * NV + b] = Fk[a].d[b];
+    eg::euler_flux_jac<DIM>(g, qm, dir, sA + (((size_t)k * Np + m) * NV) * NV);
   }
   __syncthreads();
   T* dst = diag + (size_t)e * n * n;
@@ -469,6 +509,52 @@ __global__ void k_couple_jac(DevMesh md, const T* __restrict__ dF, T* __restrict
   cpl[t] = side == 0 ? -acc : acc;
 }
 
+// The same blocks for NF face nodes known at compile time: a thread owns a
+// column (s', b) of a block, forms r_i(s') dF_i[a][b] once and walks the rows,
+// so an entry costs NF multiply-adds (k_couple_jac: 2 Nf and the index
+// arithmetic) and the stores of a warp stay consecutive.  Evaluation of 8,192
+// triangles p=3 with k_couple_jac and with this: 410 and 362 us in FP64, 156
+// and 87 us in FP32; Omega p=3 1305 and 973, 652 and 212 us; never slower by
+// more than 0.5% at 338 triangles.
+template <int DIM, int NF, typename T>
+__global__ void k_couple_jac_col(DevMesh md, const T* __restrict__ dF, T* __restrict__ cpl) {
+  constexpr int NV = DIM + 2;
+  const int S = md.S, nb = S * NV;
+  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (t >= 2LL * nb * md.I) return;
+  const int blk = (int)(t / nb), col = (int)(t - (int64_t)blk * nb);
+  const int nI = blk >> 1, side = blk & 1;
+  const int sp = col / NV, b = col - sp * NV;
+  const int* itf = md.ifaces + 5 * nI;
+  const int fr = itf[2 + side], fc = itf[3 - side];  // faces of the row and column elements
+  const int* nbp = md.nbrperm + itf[4] * NF;
+  const T* D = dF + ((size_t)nI * NF) * 2 * NV * NV + (side ? 0 : NV * NV) + b;
+  T P[NF][NV];
+#pragma unroll
+  for (int i = 0; i < NF; ++i) {
+    const T r = T(md.interp[((size_t)fc * NF + (side ? i : nbp[i])) * S + sp]);
+#pragma unroll
+    for (int a = 0; a < NV; ++a) P[i][a] = (side ? r : -r) * D[(size_t)i * 2 * NV * NV + a * NV];
+  }
+  const double* L[NF];
+#pragma unroll
+  for (int i = 0; i < NF; ++i) L[i] = md.liftS + ((size_t)fr * NF + (side ? nbp[i] : i)) * S;
+  T* dst = cpl + (size_t)blk * nb * nb + col;
+  for (int s = 0; s < S; ++s) {
+    T v[NV];
+#pragma unroll
+    for (int a = 0; a < NV; ++a) v[a] = T(0);
+#pragma unroll
+    for (int i = 0; i < NF; ++i) {
+      const T l = T(L[i][s]);
+#pragma unroll
+      for (int a = 0; a < NV; ++a) v[a] += l * P[i][a];
+    }
+#pragma unroll
+    for (int a = 0; a < NV; ++a) dst[(size_t)(s * NV + a) * nb] = v[a];
+  }
+}
+
 template <typename T>
 int launch_jac(eg_lo* lo, const double* q) {
   eg_mesh* m = lo->mesh;
@@ -482,8 +568,17 @@ int launch_jac(eg_lo* lo, const double* q) {
   const size_t fixed = sizeof(T) * ((size_t)m->dim * m->Np * m->nv * m->nv + (size_t)m->dim * m->Np * m->Np);
   const int gblk = fixed + sizeof(T) * (size_t)n * n > 200 * 1024 ? 1 : 0;
   const size_t smem = fixed + (gblk ? 0 : sizeof(T) * (size_t)n * n);
-  eg_phase_begin(m, EG_PHASE_OTHER);
+  // face tables of the dense faces where they fit beside it
+  const size_t faces = sizeof(T) * (size_t)m->F * m->Nf * ((size_t)m->S * m->S + m->nv * m->nv);
+  const int tabs = smem + faces <= 200 * 1024 ? 1 : 0;
+  const size_t smem_dense = smem + (tabs ? faces : 0);
+  // a thread per row and node: blocks no wider than the work, so that enough of
+  // them are resident (8,192 triangles p=1 FP64, the whole evaluation: 219 us
+  // with blocks of 256, 176 with 64; p=3: 417 with 256, 384 with 128; 72
+  // unknowns p=4: 774 with 128, 696 with 256)
+  const int threads = n * m->Np <= 64 ? 64 : n * m->Np <= 600 ? 128 : 256;
   const bool split = m->params.volume_integral_type == 2;
+  eg_phase_begin(m, EG_PHASE_OTHER);
   if (m->dim == 2) {
     k_face_jac<2, T><<<(nslot + 127) / 128, 128, 0, m->stream>>>(md, q, dF);
     if (split) {
@@ -491,10 +586,12 @@ int launch_jac(eg_lo* lo, const double* q) {
       k_elem_jac_split<2, T><<<m->E, 256, smem, m->stream>>>(md, q, dF, diag, gblk);
     } else if (m->sparse_face) {
       cudaFuncSetAttribute(k_elem_jac_diag<2, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      // leave the stores an L1: 10,368 tets p=2 in FP32 374 us at full residency, 351 so
+      cudaFuncSetAttribute(k_elem_jac_diag<2, T>, cudaFuncAttributePreferredSharedMemoryCarveout, 75);
       k_elem_jac_diag<2, T><<<m->E, 128, fixed, m->stream>>>(md, q, dF, diag);
     } else {
       cudaFuncSetAttribute(k_elem_jac<2, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      k_elem_jac<2, T><<<m->E, 256, smem, m->stream>>>(md, q, dF, diag, gblk);
+      k_elem_jac<2, T><<<m->E, threads, smem_dense, m->stream>>>(md, q, dF, diag, gblk, tabs);
     }
   } else {
     k_face_jac<3, T><<<(nslot + 127) / 128, 128, 0, m->stream>>>(md, q, dF);
@@ -503,10 +600,11 @@ int launch_jac(eg_lo* lo, const double* q) {
       k_elem_jac_split<3, T><<<m->E, 256, smem, m->stream>>>(md, q, dF, diag, gblk);
     } else if (m->sparse_face) {
       cudaFuncSetAttribute(k_elem_jac_diag<3, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      cudaFuncSetAttribute(k_elem_jac_diag<3, T>, cudaFuncAttributePreferredSharedMemoryCarveout, 75);
       k_elem_jac_diag<3, T><<<m->E, 128, fixed, m->stream>>>(md, q, dF, diag);
     } else {
       cudaFuncSetAttribute(k_elem_jac<3, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      k_elem_jac<3, T><<<m->E, 256, smem, m->stream>>>(md, q, dF, diag, gblk);
+      k_elem_jac<3, T><<<m->E, threads, smem_dense, m->stream>>>(md, q, dF, diag, gblk, tabs);
     }
   }
   const int64_t ncpl = (int64_t)eg_lo_coupling_size(lo);
@@ -517,6 +615,14 @@ int launch_jac(eg_lo* lo, const double* q) {
         k_couple_jac_diag<2, T><<<blocks, 256, 0, m->stream>>>(md, dF, cpl);
       else
         k_couple_jac_diag<3, T><<<blocks, 256, 0, m->stream>>>(md, dF, cpl);
+    } else if (m->dim == 2 && m->Nf >= 2 && m->Nf <= 5) {
+      const int cb = (int)((2LL * m->S * m->nv * m->I + 127) / 128);
+      switch (m->Nf) {  // Gauss faces of degree 1 to 4
+        case 2: k_couple_jac_col<2, 2, T><<<cb, 128, 0, m->stream>>>(md, dF, cpl); break;
+        case 3: k_couple_jac_col<2, 3, T><<<cb, 128, 0, m->stream>>>(md, dF, cpl); break;
+        case 4: k_couple_jac_col<2, 4, T><<<cb, 128, 0, m->stream>>>(md, dF, cpl); break;
+        default: k_couple_jac_col<2, 5, T><<<cb, 128, 0, m->stream>>>(md, dF, cpl);
+      }
     } else if (m->dim == 2) {
       k_couple_jac<2, T><<<blocks, 256, 0, m->stream>>>(md, dF, cpl);
     } else {

@@ -210,6 +210,42 @@ __device__ __forceinline__ void euler_flux(const Gas& g, const T* q, const Tn* d
   }
 }
 
+// A[a][b] = d(F . dir)_a / dq_b in closed form, fewer FP64 instructions than
+// euler_flux over Fwd: with velocity u, U = u.dir, H = (E + p)/rho and
+// phi = (gamma-1) |u|^2 / 2,
+//   mass      [ 0,                dir_j,                                       0      ]
+//   momentum  [ phi dir_i - u_i U, u_i dir_j + U delta_ij - (gamma-1) u_j dir_i, (gamma-1) dir_i ]
+//   energy    [ U (phi - H),      H dir_j - (gamma-1) u_j U,                   gamma U ]
+template <int DIM, typename T>
+__device__ __forceinline__ void euler_flux_jac(const Gas& g, const T* q, const T* dir, T* A) {
+  constexpr int NV = DIM + 2;
+  const T g1 = T(g.gamma_1), r = rcp_(q[0]);
+  T u[DIM], U = T(0), v2 = T(0);
+#pragma unroll
+  for (int i = 0; i < DIM; ++i) {
+    u[i] = q[1 + i] * r;
+    U += u[i] * dir[i];
+    v2 += u[i] * u[i];
+  }
+  const T phi = T(0.5) * g1 * v2;
+  const T H = T(g.gamma) * (q[NV - 1] * r) - phi;
+  A[0] = T(0);
+  A[NV - 1] = T(0);
+#pragma unroll
+  for (int j = 0; j < DIM; ++j) {
+    const T gu = g1 * u[j];
+    A[1 + j] = dir[j];
+#pragma unroll
+    for (int i = 0; i < DIM; ++i)
+      A[(1 + i) * NV + 1 + j] = u[i] * dir[j] - gu * dir[i] + (i == j ? U : T(0));
+    A[(NV - 1) * NV + 1 + j] = H * dir[j] - gu * U;
+    A[(1 + j) * NV] = phi * dir[j] - u[j] * U;
+    A[(1 + j) * NV + NV - 1] = g1 * dir[j];
+  }
+  A[(NV - 1) * NV] = U * (phi - H);
+  A[NV * NV - 1] = T(g.gamma) * U;
+}
+
 // Roe flux: F(qL).n + 0.5 (|A_hat| - A_hat)(qL - qR), eigenvalue floors 0.025.
 // Arranged to spend one division (FP64 is the scarce resource on GB300):
 // 1/(sqL + sqR).  Four reciprocal square roots give the rest:
