@@ -63,9 +63,9 @@ __device__ __forceinline__ Limbs to_limbs(double x, int ex) {
 }
 
 template <int DIM>
-__global__ void k_split_element(DevMesh md, const double* __restrict__ q,
-                                const double* __restrict__ fflux, Epilogue ep,
-                                unsigned int* __restrict__ status, int epb) {
+__device__ __forceinline__ void split_element(const DevMesh& md, const double* __restrict__ q,
+                                              const double* __restrict__ fflux, const Epilogue& ep,
+                                              unsigned int* __restrict__ status, int epb) {
   constexpr int NV = DIM + 2;
   constexpr int F = DIM + 1;
   constexpr int D2 = DIM * DIM;
@@ -209,6 +209,44 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q,
   write_residual<NV>(ep, sres, (size_t)e0 * Np * NV, nloc * Np * NV);
 }
 
+template <int DIM>
+__global__ void k_split_element(DevMesh md, const double* __restrict__ q, const double* __restrict__ fflux,
+                                Epilogue ep, unsigned int* __restrict__ status, int epb) {
+  split_element<DIM>(md, q, fflux, ep, status, epb);
+}
+
+// The pair loop takes 114 registers (84 on triangles), too many for a block of
+// more than 544 (736) threads to launch.  Wider blocks, which only an explicit
+// launch configuration or the autotuner asks for, run a build held to the
+// registers that MAXT threads leave.
+template <int DIM, int MAXT>
+__global__ void __launch_bounds__(MAXT) k_split_wide(DevMesh md, const double* __restrict__ q,
+                                                     const double* __restrict__ fflux, Epilogue ep,
+                                                     unsigned int* __restrict__ status, int epb) {
+  split_element<DIM>(md, q, fflux, ep, status, epb);
+}
+
+template <int DIM>
+int launch_split(eg_mesh* m, const DevMesh& md, const double* q, const Epilogue& ep, int epb, int threads,
+                 size_t smem) {
+  // once per process (thread-safe static initialisation)
+  static const int narrow = [] {
+    cudaFuncSetAttribute(k_split_element<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_split_wide<DIM, 768>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(k_split_wide<DIM, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, k_split_element<DIM>) == cudaSuccess ? a.maxThreadsPerBlock : 0;
+  }();
+  const int blocks = (m->E + epb - 1) / epb;
+  if (threads <= narrow)
+    k_split_element<DIM><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
+  else if (threads <= 768)
+    k_split_wide<DIM, 768><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
+  else
+    k_split_wide<DIM, 1024><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
+  return EG_OK;
+}
+
 }  // namespace
 
 int eg_launch_split_element(eg_mesh* m, const double* q, const Epilogue& ep, int epb) {
@@ -217,17 +255,6 @@ int eg_launch_split_element(eg_mesh* m, const double* q, const Epilogue& ep, int
   size_t smem;
   const int st = eg_element_shape(m, epb, 0, &threads, &smem);
   if (st != EG_OK) return st;
-  const int blocks = (m->E + epb - 1) / epb;
-  // once per process (thread-safe static initialisation)
-  static const bool attr_set = [] {
-    cudaFuncSetAttribute(k_split_element<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_split_element<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return true;
-  }();
-  (void)attr_set;
-  if (m->dim == 2)
-    k_split_element<2><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
-  else
-    k_split_element<3><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);
-  return EG_OK;
+  return m->dim == 2 ? launch_split<2>(m, md, q, ep, epb, threads, smem)
+                     : launch_split<3>(m, md, q, ep, epb, threads, smem);
 }

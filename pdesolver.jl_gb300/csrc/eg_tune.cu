@@ -119,6 +119,7 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
     m->vol_mma = cand[k].volume_mma;
     st = eg_launch_element(m, q_dev, res);  // warm-up (instruction cache, attributes)
     if (st != EG_OK) break;
+    if (cudaGetLastError() != cudaSuccess) continue;  // this shape does not launch: no time to compare
     cudaEventRecord(ev0, m->stream);
     for (int r = 0; r < reps && st == EG_OK; ++r) st = eg_launch_element(m, q_dev, res);
     cudaEventRecord(ev1, m->stream);

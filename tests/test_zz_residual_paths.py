@@ -84,3 +84,29 @@ def test_split_form_on_uneven_metrics_and_states(gpu_lib, oracle, dim, family, p
     ref = oracle_residual(oracle, g.desc, g.params, np.ascontiguousarray(q))
     err = np.abs(res - ref).reshape(E, -1).max(1)
     assert np.all(err <= 1e-12 * np.abs(ref).reshape(E, -1).max(1))
+
+
+# blocks of the narrow, the middle and the widest build of the split kernel, and
+# the thread counts on both sides of each edge
+@pytest.mark.parametrize("dim,p,epbs", [(3, 1, (1, 50, 73, 74, 100, 146)), (3, 2, (1, 22, 23, 24, 32, 33, 44)),
+                                        (2, 2, (1, 73, 74, 109, 110, 146))])
+def test_split_form_runs_at_every_block_width(gpu_lib, oracle, dim, p, epbs):
+    if dim == 3:
+        ms, opts, q = problems.config3(n=4, p=p, seed=4)
+    else:
+        ms, opts, q = problems.config1(n=12, p=p, family="gamma", seed=4)
+        opts = dict(opts, Flux_name="IRFlux", volume_integral_type=2, Volume_flux_name="IRFlux")
+    g = eulergpu.GPUMesh(ms, opts)
+    ref = oracle_residual(oracle, g.desc, g.params, q)
+    widths = set()
+    for epb in epbs:
+        if epb * ms.sbp.numnodes > 1024:
+            continue
+        try:
+            g.set_launch_config(epb, False)
+        except eulergpu.EulerGPUError:
+            continue                         # refused for its shared memory
+        widths.add(epb * ms.sbp.numnodes)
+        r = g.eval_residual(q, np.zeros_like(q))
+        assert np.abs(r - ref).max() <= 1e-12 * np.abs(ref).max(), epb
+    assert len(widths) >= 4 and max(widths) > 512
