@@ -39,6 +39,7 @@ struct eg_ls {
   int m;           // restart length
   double reltol, abstol, dtol;
   int itermax;
+  void* mem;       // the device buffers below but G, in one allocation
   void* V;         // [(m+1)][ndof] (stream path), or (m+2) vectors of the persistent
                    // solve, block-local (eg_basis_values)
   void* w;         // [ndof]

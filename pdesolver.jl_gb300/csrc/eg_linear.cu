@@ -735,8 +735,7 @@ extern "C" int eg_pc_apply(eg_pc* pc, const double* x, double* y, int32_t mem) {
 static void ls_free(eg_ls* ls) {
   if (!ls) return;
   eg_gmres_release(ls);
-  void* bufs[] = {ls->V, ls->w, ls->z, ls->xT, ls->bT, ls->part, ls->h, ls->y, ls->xd, ls->bd,
-                  ls->dH, ls->dflags, ls->dscal, ls->cfs, ls->dargs, ls->G, ls->tpart};
+  void* bufs[] = {ls->mem, ls->dargs, ls->G};
   for (void* b : bufs)
     if (b) cudaFree(b);
   if (ls->hh) cudaFreeHost(ls->hh);
@@ -762,15 +761,44 @@ extern "C" int eg_ls_create(eg_lo* lo, eg_pc* pc, int32_t restart, eg_ls** out) 
   ls->nblk = EG_GMRES_STREAM_BLOCKS;
   const int64_t N = lo->mesh->ndof;
   const size_t es = lo->prec == EG_F64 ? 8 : 4;
-  cudaError_t e = cudaMalloc(&ls->V, es * eg_basis_values(restart, N));
-  if (e == cudaSuccess) e = cudaMalloc(&ls->w, es * N);
-  if (e == cudaSuccess) e = cudaMalloc(&ls->z, es * N);
-  if (e == cudaSuccess && lo->mesh->I) {
-    const size_t ct = eg_face_tag_bytes(lo->mesh->I, lo->nb, es), pt = eg_part_tag_bytes(es);
-    e = cudaMalloc(&ls->cfs, ct);
-    if (e == cudaSuccess) e = cudaMemset(ls->cfs, 0, ct);
-    if (e == cudaSuccess) e = cudaMalloc(&ls->tpart, pt);
-    if (e == cudaSuccess) e = cudaMemset(ls->tpart, 0, pt);
+  // one allocation for every buffer but G: an allocation and its release cost
+  // more than most of these buffers' first use (tags and flags start at zero)
+  const size_t ct = lo->mesh->I ? eg_face_tag_bytes(lo->mesh->I, lo->nb, es) : 0;
+  const size_t pt = lo->mesh->I ? eg_part_tag_bytes(es) : 0;
+  size_t end = 0;
+  auto take = [&end](size_t bytes) {
+    const size_t at = end;
+    end += (bytes + 511) & ~size_t(511);
+    return at;
+  };
+  const size_t o_cfs = take(ct), o_tpart = take(pt), o_flags = take(sizeof(int) * 16), zeroed = end;
+  const size_t o_V = take(es * eg_basis_values(restart, N)), o_w = take(es * N), o_z = take(es * N);
+  const size_t o_xT = take(es * N), o_bT = take(es * N), o_xd = take(8 * N), o_bd = take(8 * N);
+  const size_t o_part = take(es * eg_gmres_partials(restart)), o_h = take(es * 4 * (restart + 2));
+  const size_t o_y = take(es * (restart + 1)), o_scal = take(sizeof(double) * 8);
+  // Hessenberg, Givens and least-squares state in FP64: H[(m+1) m] | cs[m] |
+  // sn[m] | g[m+1] | y[m]
+  const size_t o_dH = take(sizeof(double) * ((size_t)(restart + 1) * restart + 4 * (restart + 1)));
+  cudaError_t e = cudaMalloc(&ls->mem, end);
+  if (e == cudaSuccess) {
+    char* base = (char*)ls->mem;
+    ls->cfs = ct ? base + o_cfs : nullptr;
+    ls->tpart = pt ? base + o_tpart : nullptr;
+    ls->dflags = (int*)(base + o_flags);  // flags[0..7] + two arrival counters of the fused reductions
+    ls->V = base + o_V;
+    ls->w = base + o_w;
+    ls->z = base + o_z;
+    ls->xT = base + o_xT;
+    ls->bT = base + o_bT;
+    ls->xd = (double*)(base + o_xd);
+    ls->bd = (double*)(base + o_bd);
+    ls->part = base + o_part;
+    ls->h = base + o_h;
+    ls->y = base + o_y;
+    ls->dscal = (double*)(base + o_scal);
+    ls->dH = (double*)(base + o_dH);
+    e = cudaMemsetAsync(base, 0, zeroed, lo->mesh->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(lo->mesh->stream);
   }
   // without memory for the pushed operators the solver keeps to the stream path
   if (e == cudaSuccess && lo->mesh->I && !lo->mesh->sparse_face &&
@@ -778,21 +806,6 @@ extern "C" int eg_ls_create(eg_lo* lo, eg_pc* pc, int32_t restart, eg_ls** out) 
     ls->G = nullptr;
     cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMalloc(&ls->xT, es * N);
-  if (e == cudaSuccess) e = cudaMalloc(&ls->bT, es * N);
-  if (e == cudaSuccess) e = cudaMalloc(&ls->part, es * eg_gmres_partials(restart));
-  if (e == cudaSuccess) e = cudaMalloc(&ls->h, es * 4 * (restart + 2));
-  if (e == cudaSuccess) e = cudaMalloc(&ls->y, es * (restart + 1));
-  // Hessenberg, Givens and least-squares state in FP64: H[(m+1) m] | cs[m] |
-  // sn[m] | g[m+1] | y[m]
-  if (e == cudaSuccess)
-    e = cudaMalloc((void**)&ls->dH, sizeof(double) * ((size_t)(restart + 1) * restart + 4 * (restart + 1)));
-  // flags[0..7] + two arrival counters of the fused reductions (zeroed)
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ls->dflags, sizeof(int) * 16);
-  if (e == cudaSuccess) e = cudaMemset(ls->dflags, 0, sizeof(int) * 16);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ls->dscal, sizeof(double) * 8);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ls->xd, 8 * N);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&ls->bd, 8 * N);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&ls->hh, 8 * (restart + 16));
   if (e != cudaSuccess) {
     ls_free(ls);
