@@ -97,26 +97,36 @@ def krylov_kernel_bytes(ms, es):
 def gmres_bytes(ms, its, m, es):
     """Algorithmic bytes of one GMRES(m) solve in the persistent kernel with
     `its` Arnoldi iterations (full cycles but the last), es bytes per value.
-    Arnoldi iteration j (basis v_0..v_j): the inverse blocks and the coupling
-    blocks once (the operator I + C D^-1), v_j read and w written by the
-    operator, one Gram-Schmidt pass (dots: v_0..v_j and w read; update:
-    v_0..v_j and w read, v_{j+1} written), i.e. (2 j + 7) vectors.  Per cycle:
-    the residual b - J x (element and coupling blocks, x, b, r and v_0: 5
-    vectors) and the update x += D^-1 V y (jdone + 3 vectors and the inverse
-    blocks); one more residual ends the solve.  No cache reuse is credited,
-    and the second Gram-Schmidt passes are not counted."""
-    nv = ms.numDofPerNode
-    n = ms.sbp.numnodes * nv
-    nb = ms.sbp.stencilsize * nv
+    Arnoldi iteration j (basis v_0..v_j) on the R rows that C D^-1 can reach
+    (the nodes on a face stencil; all rows where face nodes are volume nodes):
+    the operator once, v_j read and w written, one Gram-Schmidt pass (dots:
+    v_0..v_j and w read; update: v_0..v_j and w read, v_{j+1} written), i.e.
+    (2 j + 7) vectors of R rows.  The operator is the pushed one, F nb rows on
+    R columns an element, formed once a solve from the inverse and coupling
+    blocks; with face-diagonal coupling, the inverse and coupling blocks.
+    Per cycle: the residual b - J x (element and coupling blocks, x, b, r and
+    v_0: 5 vectors) and the update x += D^-1 V y (jdone + 3 vectors and the
+    inverse blocks); one more residual ends the solve.  No cache reuse is
+    credited, and the second Gram-Schmidt passes are not counted."""
+    nv, sbp = ms.numDofPerNode, ms.sbp
+    n = sbp.numnodes * nv
+    nb = sbp.stencilsize * nv
     N = ms.numDof
     blocks = ms.numEl * n * n
-    cpl = 2 * ms.numInterfaces * nb * nb
-    total, left = 0, its
+    if sbp.sparse_face:
+        R, cpl, setup = N, 2 * ms.numInterfaces * nb * nv, 0
+        op = blocks + cpl
+    else:
+        nbd = len(np.unique(sbp.perm)) * nv
+        R, cpl = ms.numEl * nbd, 2 * ms.numInterfaces * nb * nb
+        op = ms.numEl * sbp.numfaces * nb * nbd
+        setup = blocks + cpl + op
+    total, left = setup, its
     while left > 0:
         jd = min(m, left)
-        total += sum(blocks + cpl + (2 * j + 7) * N for j in range(jd))
+        total += sum(op + (2 * j + 7) * R for j in range(jd))
         total += blocks + cpl + 5 * N            # residual at the cycle start
-        total += blocks + (jd + 3) * N           # x += D^-1 V y
+        total += blocks + jd * R + 3 * N         # x += D^-1 V y
         left -= jd
     total += blocks + cpl + 5 * N                # final residual
     return es * total
@@ -469,7 +479,7 @@ def run_ours(args, rank, world, dist):
         return
     peaks, src = measured_peaks()
     fp64_peak = measure_fp64_peak(torch)
-    dom_name, dom_ms, dom_bytes = "k_gmres_coop", t_gm, b_gm
+    dom_name, dom_ms, dom_bytes = "k_gmres", t_gm, b_gm
     achieved = dom_bytes / (dom_ms * 1e-3) / 1e9
     traffic = None
     traffic_source = None
@@ -478,7 +488,7 @@ def run_ours(args, rank, world, dist):
         # kernel on the same system (profiles/), scaled to this launch
         with open(os.path.join(ROOT, "profiles", "krylov_c2_traffic.json")) as f:
             rec = json.load(f)
-        per_it = rec.get("k_gmres_coop_bytes_per_iteration")
+        per_it = rec.get("k_gmres_bytes_per_iteration")
         if per_it:
             traffic = per_it * st_gm.iters
             traffic_source = ("profiles/krylov_c2_traffic.json (captured %s): %s; DRAM bytes per "
@@ -537,6 +547,9 @@ def run_ours(args, rank, world, dist):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
                      "traffic_source": traffic_source, "peak_source": src,
+                     "note": "algorithmic bytes credit no cache reuse; the operator and the basis stay "
+                             "in L2 and shared memory between iterations, so achieved can exceed the "
+                             "HBM copy rate (traffic: DRAM bytes)",
                      "kernel": dom_name + " (FP32: one launch = one GMRES(30) solve of the p=3 "
                                "Newton system at the converged state, %d iterations)" % st_gm.iters,
                      "algorithmic_bytes_per_launch": dom_bytes, "kernel_ms": dom_ms,
@@ -1304,7 +1317,7 @@ def run_kernels_only(args, which):
         x = torch.zeros_like(b)
         st = ls.solve(b, x)
         torch.cuda.synchronize()
-        out["kernels"] = ["k_gmres_cluster<2,28,float>"]
+        out["kernels"] = ["k_gmres<2,28,float>"]
         out["iterations"] = st.iters
         print(json.dumps(out), flush=True)
         return
@@ -1339,7 +1352,7 @@ def run_kernels_only(args, which):
             for _ in range(args.steps):
                 pc.calc()
             torch.cuda.synchronize()
-        out["kernels"] = ["k_block_inverse_reg<float,2,8,8>", "k_block_inverse_reg<float,4,8,16>"]
+        out["kernels"] = ["k_inverse_warp", "k_inverse_cta"]
         out["launches_each"] = args.steps
         print(json.dumps(out), flush=True)
         return

@@ -284,7 +284,7 @@ int eg_ls_set_grid(eg_ls* ls, int32_t blocks);
    window_us of each other (or as soon as every thread inside eg_newton_solve
    with such a solve has reached one) run as one cooperative launch: each
    solve keeps the blocks it gets alone, solves are packed while their blocks
-   fit on the SMs, and barriers cover a solve's own blocks only.  One-block
+   fit on the SMs, and blocks exchange tagged words within their solve only.  One-block
    solves launch at once (they share the GPU without batching).  Meant for many meshes solved at once on different threads/streams
    (batches, serving).  A solve's result does not depend on the batch it runs
    in.  Off by default. */
@@ -294,9 +294,10 @@ int eg_ls_solve(eg_ls* ls, const double* b, double* x, int32_t mem, eg_ls_stats*
 /* linearSolveTranspose (reference ls_standard.jl:230-244, the adjoint solve of
    calcAdjoint): x <- A^-T b by GMRES(restart) right-preconditioned with the
    transposed block-Jacobi inverses, on J^T M^-T = I + C^T D^-T (coupling
-   blocks applied transposed, element blocks cancel); same tolerances, device
-   Hessenberg and Givens, and restart cycles replayed as CUDA graphs as the
-   forward solve's stream path.  x is also the initial guess. */
+   blocks applied transposed, element blocks cancel); same tolerances and the
+   same persistent kernel as the forward solve, or its stream path (device
+   Hessenberg and Givens, restart cycles replayed as CUDA graphs) where the
+   persistent kernel cannot run.  x is also the initial guess. */
 int eg_ls_solve_transpose(eg_ls* ls, const double* b, double* x, int32_t mem, eg_ls_stats* stats);
 
 /* ---- Newton and RK4 drivers ------------------------------------------- */
