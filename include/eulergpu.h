@@ -279,6 +279,11 @@ int eg_ls_set_tolerances(eg_ls* ls, double reltol, double abstol, double dtol, i
    counterpart; the result does not depend on it beyond the order of the FP
    reductions. */
 int eg_ls_set_grid(eg_ls* ls, int32_t blocks);
+/* Failure detection of the persistent GMRES kernel: polls that one wait
+   between its blocks may take before the solve ends with EG_ERR_TIMEOUT (0
+   restores the default of 2^21, seconds).  x is then not a solution; the
+   solver stays usable. */
+int eg_ls_set_wait_limit(eg_ls* ls, int32_t polls);
 /* Batched persistent GMRES (process-wide switch; no reference counterpart).
    When enabled, the multi-block Krylov solves that threads reach within
    window_us of each other (or as soon as every thread inside eg_newton_solve

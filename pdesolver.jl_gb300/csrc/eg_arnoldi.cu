@@ -29,8 +29,8 @@
 // system whose element blocks take at most 2 MB or whose grid would have at
 // most 16 blocks, one thread-block cluster (co-scheduled by the hardware, so
 // the small solves of concurrent host threads run side by side).  Waits are
-// bounded: a block whose wait runs out leaves, F_DONE stays 0 and the host
-// reports EG_ERR_TIMEOUT.
+// bounded: a block whose wait runs out raises a flag that the other waits
+// sample and leaves without publishing, and the host reports EG_ERR_TIMEOUT.
 #include <mutex>
 
 #include "eg_arnoldi_launch.cuh"

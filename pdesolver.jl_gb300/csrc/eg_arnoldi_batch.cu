@@ -15,8 +15,8 @@
 // queueing for it one multi-block grid at a time.
 //
 // Every block of a cooperative launch is resident, so the waits between a
-// problem's blocks always end; each is bounded all the same, and a solve that
-// gave up leaves its F_DONE at 0, which its caller reports as EG_ERR_TIMEOUT.
+// problem's blocks always end; each is bounded all the same, and a solve with a
+// wait that ran out says so in its flags: its caller returns EG_ERR_TIMEOUT.
 #include <algorithm>
 #include <atomic>
 #include <chrono>

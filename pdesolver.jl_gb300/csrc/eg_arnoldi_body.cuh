@@ -19,8 +19,6 @@ constexpr int NT = 1024;  // one block per SM
 constexpr int NB_MAX = 64;  // coupling-block rows handled by the face-side pass
 // systems whose element blocks take at most this many bytes run on one cluster
 constexpr size_t kSmallOperatorBytes = size_t(2) << 20;
-// polls of one wait for a tagged word before the block gives up (seconds)
-constexpr int kSpinLimit = 1 << 21;
 constexpr int kLine = 16;  // words of a 128-byte line
 // dynamic shared memory of a block (227 KB less the static part)
 constexpr size_t kSmemBudget = 208 * 1024, kSmemStream = 176 * 1024;
@@ -55,6 +53,7 @@ struct CoopArgs {
   int nb, nbp, Rp;   // rows of a face side, padded to 4; rows of an element's pushes F nbp
   int nbn;           // nodes on some face stencil (dense faces; all Np with face-diagonal ones)
   int S, F, nv;
+  int polls;         // polls of one wait before its block gives up
   // shared-memory plan of the launch (plan_smem)
   int ec;            // elements of a staged chunk (face-diagonal operators)
   int fs_smem, ws, p0_smem;  // face table, work vectors, interior products in shared memory
@@ -238,7 +237,7 @@ struct GmresShared {
   T scs[32], ssn[32], sg[33], syT[33];
   T sR[32 * 33];  // rotated Hessenberg columns: sR[j * (m+1) + k]
   double sRd[sizeof(T) == 4 ? 32 * 33 : 1];  // the same in FP64, for the back substitution
-  int s_done, s_its, s_jdone, s_conv, s_cycles, s_nreorth, s_err, s_reorth;
+  int s_done, s_its, s_jdone, s_conv, s_cycles, s_nreorth, s_reorth;
   T s_beta, s_g0, s_hn, s_inv, s_a1;
   double s_tol, s_bnorm;
 };
@@ -281,16 +280,27 @@ __device__ __forceinline__ T* basis(const CoopArgs<T>& a, const BlockView<T>& v,
 // after reading those of t.
 constexpr int kDirect = 32;
 
-// poll one word until it carries the tag
+// After a poll that failed: true when the wait is over without its word.  The
+// wait that runs out of polls raises flags[F_GAVE_UP], which every wait samples,
+// so all blocks leave.  A thread that gave up waits no more, its block returns
+// at the next barrier and publishes nothing that depends on the missing word:
+// every word that carries its tag is a good one.
 template <typename T>
-__device__ __forceinline__ T word_wait(const uint64_t* p, unsigned tag, int* s_err) {
-  T val;
+__device__ __forceinline__ bool give_up(const CoopArgs<T>& a, int& polls) {
+  ++polls;
+  if (polls > a.polls) {
+    atomicExch(a.flags + F_GAVE_UP, 1);
+    return true;
+  }
+  return (polls & 255) == 0 && *(volatile int*)(a.flags + F_GAVE_UP) != 0;
+}
+
+// poll one word until it carries the tag; bad: given up
+template <typename T>
+__device__ __forceinline__ T word_wait(const CoopArgs<T>& a, const uint64_t* p, unsigned tag, bool& bad) {
+  T val = T(0);
   int polls = 0;
-  while (!msg_get(p, tag, val))
-    if (++polls > kSpinLimit) {
-      *s_err = 1;
-      break;
-    }
+  while (!bad && !msg_get(p, tag, val)) bad = give_up(a, polls);
   return val;
 }
 // publish this block's partial k of reduction `tag` (lane 0 of a warp)
@@ -299,26 +309,27 @@ __device__ __forceinline__ void part_put(const CoopArgs<T>& a, const BlockView<T
   if ((threadIdx.x & 31) == 0)
     msg_put(a.part + (size_t)(((tag & 1) * 33 + k) * v.nblk + v.b) * kWords<T>, val, tag);
 }
-// out[k] = sum over the blocks of partial k < cnt, the same bits in every block
+// out[k] = sum over the blocks of partial k < cnt, the same bits in every
+// block; true in a thread that gave up
 template <typename T>
-__device__ __forceinline__ void part_sum(const CoopArgs<T>& a, const BlockView<T>& v, int cnt, T* out, unsigned tag,
-                                         int* s_err) {
+__device__ __forceinline__ bool part_sum(const CoopArgs<T>& a, const BlockView<T>& v, int cnt, T* out, unsigned tag) {
+  bool bad = false;
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   if (v.nblk <= kDirect) {
-    if (k >= cnt) return;
+    if (k >= cnt) return false;
     const uint64_t* p = a.part + (size_t)((tag & 1) * 33 + k) * v.nblk * kWords<T>;
     T acc = T(0);
-    for (int r = lane; r < v.nblk; r += 32) acc += word_wait<T>(p + r * kWords<T>, tag, s_err);
+    for (int r = lane; r < v.nblk; r += 32) acc += word_wait(a, p + r * kWords<T>, tag, bad);
     acc = wsum(acc);
     if (lane == 0) out[k] = acc;
-    return;
+    return bad;
   }
   if (k < cnt && v.b == k * (v.nblk / 33)) {
     const uint64_t* p = a.part + (size_t)((tag & 1) * 33 + k) * v.nblk * kWords<T>;
     T acc = T(0);
     int polls = 0;
     constexpr int U = 5;
-    for (int b0 = lane; b0 < v.nblk; b0 += 32 * U) {
+    for (int b0 = lane; b0 < v.nblk && !bad; b0 += 32 * U) {
       T val[U];
       bool all;
       do {
@@ -328,19 +339,18 @@ __device__ __forceinline__ void part_sum(const CoopArgs<T>& a, const BlockView<T
           val[u] = T(0);
           if (b0 + 32 * u < v.nblk) all &= msg_get(p + (size_t)(b0 + 32 * u) * kWords<T>, tag, val[u]);
         }
-        if (!all && ++polls > kSpinLimit) {
-          *s_err = 1;
-          break;
-        }
-      } while (!all);
+        if (!all) bad = give_up(a, polls);
+      } while (!all && !bad);
 #pragma unroll
       for (int u = 0; u < U; ++u) acc += val[u];
     }
+    const bool good = !__any_sync(0xffffffffu, bad);
     acc = wsum(acc);
-    if (lane == 0) msg_put(a.tot + (size_t)((tag & 1) * 33 + k) * kLine, acc, tag);
+    if (lane == 0 && good) msg_put(a.tot + (size_t)((tag & 1) * 33 + k) * kLine, acc, tag);
   }
   if (k == 31 && lane < cnt)
-    out[lane] = word_wait<T>(a.tot + (size_t)((tag & 1) * 33 + lane) * kLine, tag, s_err);
+    out[lane] = word_wait(a, a.tot + (size_t)((tag & 1) * 33 + lane) * kLine, tag, bad);
+  return bad;
 }
 
 // partial dots of the block's rows against x: warp k < cnt takes V[k] (plus
@@ -604,10 +614,11 @@ __device__ __forceinline__ void build_push_operator(const CoopArgs<T>& a, const 
 
 // Sum of the pushed products that land on row (node j, variable av) of own
 // element le, in face order: one term per simplex face whose stencil holds the
-// node and that couples to a neighbour.  Polls until all of them carry `tag`.
+// node and that couples to a neighbour.  Polls until all of them carry `tag`;
+// bad: given up.
 template <int DIM, typename T>
 __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v, const int* sSpos, int le, int j,
-                                    int av, unsigned tag, int* s_err) {
+                                    int av, unsigned tag, bool& bad) {
   constexpr int NV = DIM + 2, FF = DIM + 1;
   const uint64_t* p[FF];
 #pragma unroll
@@ -626,11 +637,8 @@ __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v,
       val[f] = T(0);
       if (p[f]) all &= msg_get(p[f], tag, val[f]);
     }
-    if (!all && ++polls > kSpinLimit) {
-      *s_err = 1;
-      break;
-    }
-  } while (!all);
+    if (!all) bad = give_up(a, polls);
+  } while (!all && !bad);
   T acc = T(0);
 #pragma unroll
   for (int f = 0; f < FF; ++f) acc += val[f];
@@ -729,8 +737,8 @@ __host__ __device__ __forceinline__ int block_first(int64_t E, int b, int nblk) 
 // Blocks exchange the pushed face products and the dot-product partials as
 // tagged words; every block sums the partials in the same order, so the
 // scalars are bit-identical in every block and all blocks take the same
-// branches.  A block whose wait runs out leaves (flags[F_DONE] stays 0), and
-// so does every block that then waits for it.
+// branches.  A wait that runs out raises flags[F_GAVE_UP]; its block and every
+// block that waits later leave, and the host reports the solve as failed.
 template <int DIM, int NB, typename T>
 __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, GmresShared<T>& sm) {
   constexpr int NV = DIM + 2;
@@ -778,7 +786,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
   for (int k = tid; k < a.F * a.S; k += NT) sm.sPerm[k] = a.md.perm[k];
   for (int k = tid; k < a.F * Np; k += NT) sm.sSpos[k] = a.spos[k];
   if (tid == 0) {
-    sm.s_its = sm.s_cycles = sm.s_nreorth = sm.s_err = 0;
+    sm.s_its = sm.s_cycles = sm.s_nreorth = 0;
     sm.s_conv = 0;
     // nodes on some face stencil first (face-diagonal operators: all nodes)
     int q = 0;
@@ -815,8 +823,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       const T s = wsum(sm.sR[32 * wq + lane]);
       part_put(a, v, wq, s, rt);
     }
-    part_sum(a, v, 2, sm.sh1, rt, &sm.s_err);
-    __syncthreads();
+    if (__syncthreads_or(part_sum(a, v, 2, sm.sh1, rt))) return;
     if (tid == 0) {
       sm.s_bnorm = sqrt(double(sm.sh1[0]));
       sm.s_tol = fmax(a.scal[S_RELTOL] * sm.s_bnorm, a.scal[S_ABSTOL]);
@@ -825,25 +832,25 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
   bool xzero = sm.sh1[1] == T(0);
   __syncthreads();
   for (;;) {
-    if (sm.s_err) return;
     // ---- r = b - J x (natural rows, in a.w); the pushed products cross blocks
+    bool bad = false;
     if (xzero) {
       for (int t = tid; t < nat; t += NT) a.w[r0 + t] = a.bvec[r0 + t];
     } else {
       ++pt;
       couple_push<DIM, T>(a, v, a.x + r0, 0, v.nel, sm.sPerm, pt, pol);
-      for (int t = tid; t < nat; t += NT) {
+      for (int t = tid; t < nat && !bad; t += NT) {
         const int le = t / n, r = t - le * n;
         const int e = v.e0 + le;
         const T* A = a.diag + (size_t)e * n * n;
         const T* xe = a.x + (size_t)e * n;
         const T d = a.trans ? block_col<T>(A, xe, r, n) : block_row<NB, T>(A, xe, r, n);
         const int j = r / NV;
-        a.w[r0 + t] = a.bvec[r0 + t] - (d + gather<DIM, T>(a, v, sm.sSpos, le, j, r - j * NV, pt, &sm.s_err));
+        a.w[r0 + t] = a.bvec[r0 + t] - (d + gather<DIM, T>(a, v, sm.sSpos, le, j, r - j * NV, pt, bad));
       }
     }
     xzero = false;
-    __syncthreads();
+    if (__syncthreads_or(bad)) return;
     // |r|^2 of the stencil rows and of the interior rows
     {
       const int lane = tid & 31, wq = tid >> 5;
@@ -867,8 +874,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
         const T s = wsum(sm.sR[32 * wq + lane]);
         part_put(a, v, wq, s, rt);
       }
-      part_sum(a, v, 2, sm.sh1, rt, &sm.s_err);
-      __syncthreads();
+      if (__syncthreads_or(part_sum(a, v, 2, sm.sh1, rt))) return;
     }
     if (tid == 0) {
       const T b2 = sm.sh1[0] + sm.sh1[1];
@@ -885,7 +891,6 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       for (int k = 1; k <= m; ++k) sm.sg[k] = T(0);
     }
     __syncthreads();
-    if (sm.s_err) return;
     if (sm.s_done) break;
     // v_0 = r / beta: stencil rows to the basis, interior rows to vint
     {
@@ -929,20 +934,19 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       apply_push<DIM, NB, T>(a, v, a.ws ? v.cur : basis(a, v, j), sm.sal[j], sm.sPerm, pt,
                              a.md.sparse_face ? 0 : 32, pol);
       __syncthreads();
-      if (sm.s_done || sm.s_err) break;
+      if (sm.s_done) break;
       // (2) w = K v_j: the pushed products of the faces holding the row's node
-      for (int t = tid; t < nrow; t += NT) {
+      for (int t = tid; t < nrow && !bad; t += NT) {
         const int le = t / nbd, q = t - le * nbd;
         const int jn = q / NV;
-        v.sw[t] = gather<DIM, T>(a, v, sm.sSpos, le, sm.sOrd[jn], q - jn * NV, pt, &sm.s_err);
+        v.sw[t] = gather<DIM, T>(a, v, sm.sSpos, le, sm.sOrd[jn], q - jn * NV, pt, bad);
       }
       if (tid < v.nrowp - nrow) v.sw[nrow + tid] = T(0);
-      __syncthreads();
+      if (__syncthreads_or(bad)) return;
       // (3) first pass: h1 = V^T w and w.w in one reduction
       ++rt;
       dots_put<T>(a, v, v.sw, j + 1, T(0), T(0), sm.sal, rt);
-      part_sum(a, v, j + 2, sm.sh1, rt, &sm.s_err);
-      __syncthreads();
+      if (__syncthreads_or(part_sum(a, v, j + 2, sm.sh1, rt))) return;
       if (tid < 32) {
         T hh, a1;
         column_sums(sm.sh1, sm.sal, j, hh, a1);
@@ -968,8 +972,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
         __syncthreads();
         ++rt;
         dots_put<T>(a, v, v.sw, j + 1, sm.s_a1, sm.s_g0, sm.sal, rt);
-        part_sum(a, v, j + 2, sm.sh2, rt, &sm.s_err);
-        __syncthreads();
+        if (__syncthreads_or(part_sum(a, v, j + 2, sm.sh2, rt))) return;
         if (tid < 32) {
           T hh, a2;
           column_sums(sm.sh2, sm.sal, j, hh, a2);
@@ -994,7 +997,6 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
         break;
       }
     }
-    if (sm.s_err) return;
     // ---- y = R^-1 g (FP64 back substitution by warp 0), x += D^-1 V y
     const int nn = sm.s_jdone;
     if constexpr (sizeof(T) == 4) {
@@ -1104,6 +1106,7 @@ void coop_args(const eg_ls* ls, CoopArgs<T>* out) {
   a.E = m->E;
   a.N = m->ndof;
   a.trans = ls->trans;
+  a.polls = ls->polls > 0 ? ls->polls : 1 << 21;  // seconds
   a.ec = a.fs_smem = a.ws = a.p0_smem = a.kv = a.er = a.ef0 = 0;
   // evict-first operator loads when operator and Krylov basis do not fit the
   // 129 MB L2 together (the operator's lines then give way to the basis)

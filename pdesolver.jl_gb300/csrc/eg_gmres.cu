@@ -640,7 +640,7 @@ int gmres_T(eg_ls* ls, eg_ls_stats* st, int transpose) {
     EG_CUDA(cudaStreamSynchronize(m->stream));
     std::memcpy(scal, ls->hh, sizeof(scal));
     std::memcpy(flags, ls->hh + 8, sizeof(flags));
-    if (!flags[F_DONE]) return eg_gmres_gave_up(ls);
+    if (!flags[F_DONE] || flags[F_GAVE_UP]) return eg_gmres_gave_up(ls);
     if (!std::isfinite(scal[S_BETA])) {
       eg_set_error("GMRES: non-finite residual");
       return EG_ERR_NONFINITE;

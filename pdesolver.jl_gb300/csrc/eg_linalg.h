@@ -59,6 +59,7 @@ struct eg_ls {
   double* bd;      // [ndof]
   int nblk;
   int coop_grid;   // blocks of the persistent GMRES grid (0: automatic)
+  int polls;       // polls of one wait of the persistent GMRES (0: default)
   // device-side GMRES state (eg_gmres.cu)
   double* dH;      // H | cs | sn | g | y  (FP64)
   int* dflags;     // done, jdone, its, converged, itermax
@@ -82,8 +83,10 @@ struct eg_ls {
 };
 void eg_gmres_release(eg_ls* ls);
 // slots of the device GMRES state: dflags[] and dscal[]
-// (F_TAGS: two words, the last push and reduction tags of the persistent solve)
-enum { F_DONE = 0, F_JDONE = 1, F_ITS = 2, F_CONV = 3, F_ITERMAX = 4, F_REORTH = 5, F_CYCLES = 6, F_NREORTH = 7,
+// (F_TAGS: two words, the last push and reduction tags of the persistent solve;
+// F_GAVE_UP: a wait of the persistent solve ran out, in the word that the stream
+// path uses for its second pass)
+enum { F_DONE = 0, F_JDONE = 1, F_ITS = 2, F_CONV = 3, F_ITERMAX = 4, F_REORTH = 5, F_GAVE_UP = 5, F_CYCLES = 6, F_NREORTH = 7,
        F_TAGS = 12 };
 enum { S_TOL = 0, S_RESID = 1, S_BETA = 2, S_BNORM = 3, S_RELTOL = 4, S_ABSTOL = 5, S_BETA0 = 6 };
 // the whole GMRES solve as one persistent cooperative kernel (eg_arnoldi.cu)
@@ -112,8 +115,8 @@ inline size_t eg_part_tag_bytes(size_t es) { return 2 * es * 2 * 33 * (EG_COOP_M
 // before each persistent solve: reset the tagged buffers (on the mesh stream)
 // when the 32-bit tags could run out; `force` after a solve that gave up
 int eg_gmres_tags(eg_ls* ls, bool force = false);
-// a persistent solve ended without F_DONE: a wait between its blocks ran out.
-// Resets the tagged buffers and returns EG_ERR_TIMEOUT.
+// a persistent solve did not finish (no F_DONE, or F_GAVE_UP): a wait between
+// its blocks ran out.  Resets the tagged buffers and returns EG_ERR_TIMEOUT.
 int eg_gmres_gave_up(eg_ls* ls);
 int eg_gmres_coop(eg_ls* ls);
 int eg_gmres_launch_f64(eg_ls* ls);  // its FP64 launches (eg_arnoldi_f64.cu)

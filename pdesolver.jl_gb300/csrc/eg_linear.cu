@@ -824,6 +824,15 @@ extern "C" int eg_ls_set_grid(eg_ls* ls, int32_t blocks) {
   return EG_OK;
 }
 
+extern "C" int eg_ls_set_wait_limit(eg_ls* ls, int32_t polls) {
+  if (!ls || polls < 0) {
+    eg_set_error("eg_ls_set_wait_limit: invalid argument");
+    return EG_ERR_INVALID;
+  }
+  ls->polls = polls;
+  return EG_OK;
+}
+
 extern "C" int eg_ls_destroy(eg_ls* ls) {
   if (!ls) return EG_OK;
   cudaStreamSynchronize(ls->lo->mesh->stream);

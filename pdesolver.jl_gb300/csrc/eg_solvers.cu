@@ -371,16 +371,18 @@ IterOut newton_graph_iteration(eg_mesh* m, eg_newton_ws* w, double tau_l) {
   r.step = m->h_red[1];
   r.norm = m->h_red[0];
   const unsigned int status = *m->h_status;
+  const bool gave_up = !flags[F_DONE] || flags[F_GAVE_UP];
   if (status & EG_DEV_LU_PIVOT) {
     // the eager path stops before the update: put q back
     cudaMemcpyAsync(w->qd, w->qsave, 8 * m->ndof, cudaMemcpyDeviceToDevice, s);
+    if (gave_up) eg_gmres_gave_up(ls);  // the solver stays usable
     cudaStreamSynchronize(s);
     eg_set_error("zero pivot in block LU");
     r.st = EG_ERR_LU_PIVOT;
     r.updated = false;
     return r;
   }
-  if (!flags[F_DONE]) {
+  if (gave_up) {
     cudaMemcpyAsync(w->qd, w->qsave, 8 * m->ndof, cudaMemcpyDeviceToDevice, s);
     cudaStreamSynchronize(s);
     r.st = eg_gmres_gave_up(ls);

@@ -82,6 +82,7 @@ def _declare(lib):
     lib.eg_ls_solve.argtypes = [vp, vp, vp, C.c_int32, C.POINTER(LsStats)]
     lib.eg_ls_solve_transpose.argtypes = [vp, vp, vp, C.c_int32, C.POINTER(LsStats)]
     lib.eg_ls_set_grid.argtypes = [vp, C.c_int32]
+    lib.eg_ls_set_wait_limit.argtypes = [vp, C.c_int32]
     lib.eg_set_gmres_batching.argtypes = [C.c_int32, C.c_double]
     lib.eg_newton_solve.argtypes = [vp, vp, C.c_int32, C.POINTER(NewtonOpts), C.POINTER(NewtonStats)]
     lib.eg_rk4.argtypes = [vp, vp, C.c_double, C.c_double, C.c_int32, C.c_double, C.c_int32,
@@ -602,6 +603,11 @@ class LinearSolver:
     def set_grid(self, blocks=0):
         """blocks of the persistent GMRES kernel (0: automatic)."""
         check(self.lib.eg_ls_set_grid(self.handle, int(blocks)))
+
+    def set_wait_limit(self, polls=0):
+        """polls of one wait between the persistent kernel's blocks before a
+        solve fails with EG_ERR_TIMEOUT (0: the default)."""
+        check(self.lib.eg_ls_set_wait_limit(self.handle, int(polls)))
 
     def solve(self, b, x):
         pb, mb = GPUMesh._ptr(b, self.lo.g.ndof)
