@@ -171,11 +171,8 @@ class SteadySolveServer:
     slots: requests on the device at once (one host thread and CUDA stream
     each).  precision: 1 mixed (FP32 Jacobian, PC, Krylov), 0 plain FP64.
 
-    batch_gmres: the Krylov solves of requests that run at the same time share
-    launches.  A request alone shares nothing, so an idle server then starts
-    one when a second has arrived, or batch_wait seconds after its arrival (a
-    small solve takes 5 to 20 ms, less than most arrival gaps); a server with
-    requests running admits at once.
+    batch_gmres: the multi-block Krylov solves of requests that run at the
+    same time share launches.
 
     run_request / make_meshes / close_meshes / make_stream are the device
     hooks; tests replace them to check the scheduling on the CPU.
@@ -183,7 +180,7 @@ class SteadySolveServer:
 
     def __init__(self, hbm_budget, slots=8, precision=1, retries=2, max_bypass=8,
                  run_request=None, make_meshes=None, close_meshes=None, make_stream=None,
-                 clock=time.perf_counter, batch_gmres=False, batch_wait=0.03):
+                 clock=time.perf_counter, batch_gmres=False):
         self.budget = int(hbm_budget)
         self.slots = int(slots)
         self.precision = int(precision)
@@ -191,7 +188,6 @@ class SteadySolveServer:
         self.max_bypass = int(max_bypass)
         self.clock = clock
         self.batch_gmres = bool(batch_gmres) and run_request is None
-        self.batch_wait = float(batch_wait)
         self._run_request = run_request or self._gpu_run_request
         self._make_meshes = make_meshes or self._gpu_make_meshes
         self._close_meshes = close_meshes or self._gpu_close_meshes
@@ -303,18 +299,10 @@ class SteadySolveServer:
                 return k
         return None
 
-    def _companion_wait(self):
-        """seconds the only request of an idle batching server still waits for
-        a second one; called with the lock held"""
-        if (not self.batch_gmres or self._closed or self._running > 0 or len(self._pending) != 1
-                or self._pending[0].snapshot is not None):
-            return 0.0
-        return self._results[self._pending[0].rid].arrival + self.batch_wait - self.clock()
-
     def _admit(self):
         """called with the lock held: admit one request if possible; returns
         (req, meshes or None, evicted list) or None."""
-        if self._running >= self.slots or not self._pending or self._companion_wait() > 0:
+        if self._running >= self.slots or not self._pending:
             return None
         k = self._pick()
         if k is None:
@@ -349,8 +337,7 @@ class SteadySolveServer:
                     got = self._admit()
                     if got is not None:
                         break
-                    hold = self._companion_wait()
-                    self._cv.wait(hold if 0 < hold < 0.05 else 0.05)
+                    self._cv.wait(0.05)
             req, meshes, evicted = got
             for m in evicted:
                 self._close_meshes(m)
