@@ -66,8 +66,8 @@ struct eg_mesh {
   int32_t* perm;    // [F][S]
   int32_t* nbrperm; // [norient][Nf]
   double* wface;    // [Nf]
-  int32_t* Qpair;   // [2][Np/2][dim][Np][2] fixed-point Q entries of the split form's pairs
-  int Qexp;         // their scale: 2^Qexp > max |Q|
+  int32_t* Qpair;   // [2][Np/2][dim][Np][2] fixed-point Q entries of the split form's pairs,
+                    // [Np/2][Np] their scales (2^scale > the pair's largest |Q|)
   double* liftS;    // [F][Nf][S]: interp[f][i][s] * wface[i]
   int32_t* nbrinv;  // [norient][Nf]: inverse permutations of nbrperm
   int sparse_face;  // interp is the identity on every face (diagonal-E operators)

@@ -13,7 +13,7 @@ struct DevMesh {
   const int* perm;        // [F][S]
   const int* nbrperm;     // [norient][Nf]
   const int2* Qpair;      // [2][Np/2][dim][Np]: Q_m(j, j + s), Q_m(j + s, j) (indices mod Np) in fixed point
-  int Qexp;               // 2^Qexp > max |Q|
+  const int* Qexp;        // [Np/2][Np]: 2^Qexp > the pair's largest |Q|
   const double* dxidx;    // [E][Np][dim][dim]
   const int* ifaces;      // [I][5]
   const double* nrm_face; // [I][Nf][dim]

@@ -55,7 +55,7 @@ extern "C" int eg_estimate_mem(const eg_mem_query* qy, eg_mem_estimate* out) {
   mesh.add(4 * F * S);               // perm
   mesh.add(4 * no * Nf);             // nbrperm
   mesh.add(8 * Nf);                  // wface
-  mesh.add(8 * 2 * (Np / 2) * d * Np);  // Qpair
+  mesh.add(8 * 2 * (Np / 2) * d * Np + 4 * (Np / 2) * Np);  // Qpair and its scales
   mesh.add(8 * F * Nf * S);          // liftS
   mesh.add(4 * no * Nf);             // nbrinv
   mesh.add(8 * E * Np * d * d);      // dxidx

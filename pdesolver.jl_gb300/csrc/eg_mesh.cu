@@ -282,22 +282,30 @@ extern "C" int eg_mesh_create(const eg_mesh_desc* d, const eg_params* params, eg
       for (int s = 0; s < S; ++s)
         liftS[((size_t)f * Nf + i) * S + s] = d->interp[((size_t)f * Nf + i) * S + s] * d->wface[i];
   // Q entries of the split form's node pairs (j, j + s mod Np), s = 1 .. Np/2,
-  // as 60-bit fixed point relative to 2^Qexp > max |Q| (eg_split.cu)
+  // as 60-bit fixed point relative to a power of two above the pair's largest
+  // entry (eg_split.cu), followed by the exponents of these scales
   const int H = Np / 2;
-  double qmax = 0.0;
-  for (int k = 0; k < dim * Np * Np; ++k) qmax = std::fmax(qmax, std::fabs(d->Q[k]));
-  m->Qexp = qmax > 0.0 && std::isfinite(qmax) ? std::ilogb(qmax) + 1 : 1;
-  std::vector<int32_t> Qpair((size_t)2 * H * dim * Np * 2);
-  for (int t = 0; t < H * dim * Np; ++t) {
-    const int s = t / (dim * Np), k = (t / Np) % dim, j = t % Np, o = (j + s + 1) % Np;
-    for (int side = 0; side < 2; ++side) {  // Q_k(j, o), Q_k(o, j)
-      const double x = d->Q[((size_t)k * Np + (side ? j : o)) * Np + (side ? o : j)];
-      const long long v = std::isfinite(x) ? std::llrint(std::ldexp(x, 59 - m->Qexp)) : 0;
-      int32_t* q = Qpair.data() + ((size_t)side * H * dim * Np + t) * 2;
-      q[0] = (int32_t)(v >> 30);
-      q[1] = (int32_t)(v & 0x3fffffff);
+  std::vector<int32_t> Qpair((size_t)2 * H * dim * Np * 2 + (size_t)H * Np);
+  auto Qjo = [&](int k, int side, int j, int o) {  // Q_k(j, o), Q_k(o, j)
+    return d->Q[((size_t)k * Np + (side ? j : o)) * Np + (side ? o : j)];
+  };
+  for (int s = 0; s < H; ++s)
+    for (int j = 0; j < Np; ++j) {
+      const int o = (j + s + 1) % Np;
+      double qmax = 0.0;
+      for (int k = 0; k < 2 * dim; ++k) qmax = std::fmax(qmax, std::fabs(Qjo(k / 2, k % 2, j, o)));
+      const int ex = qmax > 0.0 && std::isfinite(qmax) ? std::ilogb(qmax) + 1 : 0;
+      Qpair[(size_t)4 * H * dim * Np + (size_t)s * Np + j] = ex;
+      for (int k = 0; k < dim; ++k)
+        for (int side = 0; side < 2; ++side) {
+          const double x = Qjo(k, side, j, o);
+          const long long v = std::isfinite(x) ? std::llrint(std::ldexp(x, 59 - ex)) : 0;
+          const long long h = (v + (1 << 29)) >> 30;
+          int32_t* q = Qpair.data() + (((size_t)(side * H + s) * dim + k) * Np + j) * 2;
+          q[0] = (int32_t)h;
+          q[1] = (int32_t)(v - (h << 30));
+        }
     }
-  }
   std::vector<int32_t> nbrinv((size_t)m->norient * Nf);
   for (int o = 0; o < m->norient; ++o)
     for (int i = 0; i < Nf; ++i) nbrinv[(size_t)o * Nf + d->nbrperm[o * Nf + i]] = i;

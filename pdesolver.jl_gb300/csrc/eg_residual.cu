@@ -381,7 +381,9 @@ DevMesh dev_mesh(const eg_mesh* m) {
   d.gamma = m->dp.gamma; d.gamma_1 = m->dp.gamma_1;
   d.face_flux = m->params.face_flux;
   d.Q = m->Q; d.interp = m->interp; d.perm = m->perm; d.nbrperm = m->nbrperm;
-  d.Qpair = reinterpret_cast<const int2*>(m->Qpair); d.Qexp = m->Qexp; d.dxidx = m->dxidx; d.ifaces = m->ifaces; d.nrm_face = m->nrm_face;
+  d.Qpair = reinterpret_cast<const int2*>(m->Qpair);
+  d.Qexp = m->Qpair + (size_t)4 * (m->Np / 2) * m->dim * m->Np;
+  d.dxidx = m->dxidx; d.ifaces = m->ifaces; d.nrm_face = m->nrm_face;
   d.bfaces = m->bfaces; d.nrm_bndry = m->nrm_bndry; d.qg_bndry = m->qg_bndry; d.bc_of_b = m->bc_of_b;
   d.eface = m->eface; d.Minv = m->Minv; d.w = m->w; d.jac = m->jac;
   d.liftS = m->liftS; d.nbrinv = m->nbrinv; d.wface = m->wface; d.sparse_face = m->sparse_face;
@@ -431,8 +433,7 @@ int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* s
   if (split) {
     // pair tables of both orientations, node quantities, residual
     const size_t nd = 7 + (size_t)m->dim * m->dim;
-    *smem = sizeof(double) * (2 * (size_t)(Np / 2) * m->dim * Np + lift + (size_t)epb * Np * (nd + nv)) +
-            sizeof(int) * (((size_t)epb + 1) & ~(size_t)1);
+    *smem = sizeof(double) * (2 * (size_t)(Np / 2) * m->dim * Np + lift + (size_t)epb * Np * (nd + nv));
     *threads = epb * Np;
   } else {
     *smem = sizeof(double) * ((size_t)m->dim * Np * Np + lift + (size_t)epb * (m->dim + 1) * Np * nv);

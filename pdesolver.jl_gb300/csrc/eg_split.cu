@@ -21,20 +21,24 @@
 // the other node's quantities without bank conflicts.
 //
 // The directions n_jk (18 multiply-adds per pair) are formed in the integer
-// pipe, which has room: metrics and Q entries as 60-bit fixed-point numbers
-// relative to the element's largest metric term and the largest |Q|, in two
-// 30-bit limbs; n_jk = sum of 2 DIM products, high x high and the two cross
-// terms in 64-bit accumulators (the low x low terms are below 2^-57 of full
-// scale), converted to FP64 once.  56 bits doubled the error of the residual
-// against 64-bit arithmetic; with 60 it is that of FP64 directions.  G is linear in n_jk, so
-// the scale is applied to the finished row.
+// pipe, which has room: metrics and Q entries as 60-bit fixed-point numbers in
+// two 30-bit limbs, a physical direction's metrics relative to the largest of
+// that direction in the element, a pair's Q entries relative to its largest;
+// n_jk[d] = sum of 2 DIM products, high x high and the two cross terms in
+// 64-bit accumulators, converted to FP64 once and scaled by its power of two.
+// With R and Qj the largest entries, the roundings of the inputs (2 DIM 2^-60
+// each), the low x low terms (at most 2 DIM 2^-60: the low limb is signed) and
+// the last shift sum to at most (6 DIM + 1) 2^-60 R Qj, 2^-55.7 in 3-D; FP64
+// directions round at 2^-53 of each term.  Scales of their own keep a thin
+// direction of a stretched element at that accuracy: with one scale for the
+// element an aspect ratio r cost its residual a factor r / 8.
 //
 // Bound: the FP64 pipe.  A pair costs 69 FP64 instructions (the averages from
 // the per-node quantities with two approximate reciprocals, see
 // ir_average_pre); 117 with a division, four threshold tests and separate
 // means, and a table of all pair fluxes in shared memory (17 KB per element,
 // one CTA per SM).  82,944 tets p=2, residual: 6.72 -> 3.81 ms with n_jk in
-// FP64, 3.42 ms in fixed point.
+// FP64, 3.43 ms in fixed point.
 #include "eg_internal.h"
 #include "eg_kernels.cuh"
 #include "eg_physics.cuh"
@@ -43,23 +47,32 @@ using eg::Gas;
 
 namespace {
 
-// Fixed point: round(x 2^(59 - ex)), |x| < 2^ex, as high limb (signed, 30
-// bits) and low limb (30 bits).
+// Fixed point: v = round(x 2^(59 - ex)), |x| < 2^ex, as v = h 2^30 + l with
+// |h| <= 2^29 and -2^29 <= l < 2^29.
 struct Limbs {
   int h, l;
 };
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-// smallest e with |x| < 2^e for the largest high word of |x| (normal range; 0
-// and subnormals count as 2^-1022, infinities and NaN as 2^1024)
+// smallest e with |x| < 2^e for the largest high word of |x| (normal range;
+// subnormals count as 2^-1022, infinities and NaN as 2^1024, zero as 1)
 __device__ __forceinline__ int exponent_above(int hi) {
   const int b = (hi >> 20) & 0x7ff;
-  return (b < 1 ? 1 : b) - 1022;
+  return hi == 0 ? 0 : (b < 1 ? 1 : b) - 1022;
 }
 __device__ __forceinline__ Limbs to_limbs(double x, int ex) {
   // two exact scalings: 59 - ex may exceed the exponent range of one
   const int k = 59 - ex, k1 = k / 2;
   const long long v = __double2ll_rn(x * pow2(k1) * pow2(k - k1));
-  return Limbs{(int)(v >> 30), (int)(v & 0x3fffffff)};
+  const int h = (int)((v + (1 << 29)) >> 30);
+  return Limbs{h, (int)(v - ((long long)h << 30))};
+}
+// v 2^k: the exponent field takes k (v = 0 has none), or beyond its range three
+// products
+__device__ __forceinline__ double scaled(long long v, int k) {
+  const double x = (double)v;
+  if (abs(k) <= 900) return v == 0 ? 0.0 : __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+  const int k3 = k / 3;
+  return x * pow2(k3) * pow2(k3) * pow2(k - 2 * k3);
 }
 
 template <int DIM>
@@ -80,9 +93,10 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
   double* sN = sL + F * Nf * S + (F * S + 1) / 2;  // [7][rows]: IR quantities
   Limbs* sD = reinterpret_cast<Limbs*>(sN + (size_t)7 * rows);  // [DIM DIM][rows]: metrics
   double* sres = reinterpret_cast<double*>(sD + (size_t)D2 * rows);  // [epb][Np][NV]
-  int* sMax = reinterpret_cast<int*>(sres + (size_t)rows * NV);  // [epb] largest high word of |dxidx|
-  for (int k = threadIdx.x; k < epb; k += blockDim.x) sMax[k] = 0;
-  const int exQ = md.Qexp;
+  // [epb][DIM] largest high word of |dxidx| of a physical direction, where the
+  // logarithms go later
+  int* sMax = reinterpret_cast<int*>(sN + (size_t)2 * rows);
+  for (int k = threadIdx.x; k < epb * DIM; k += blockDim.x) sMax[k] = 0;
   for (int k = threadIdx.x; k < 2 * H * DIM * Np; k += blockDim.x) {
     const int2 v = md.Qpair[k];
     sQa[k] = Limbs{v.x, v.y};
@@ -113,13 +127,16 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
 #pragma unroll
     for (int c = 0; c < NV; ++c) qj[c] = src[c];
     const double* dxj = md.dxidx + ((size_t)e0 * Np + t) * D2;
-    int hi = 0;
 #pragma unroll
-    for (int c = 0; c < D2; ++c) {
-      dxd[c] = dxj[c];
-      hi = max(hi, __double2hiint(dxd[c]) & 0x7fffffff);
+    for (int d = 0; d < DIM; ++d) {
+      int hi = 0;
+#pragma unroll
+      for (int m = 0; m < DIM; ++m) {
+        dxd[d * DIM + m] = dxj[d * DIM + m];
+        hi = max(hi, __double2hiint(dxd[d * DIM + m]) & 0x7fffffff);
+      }
+      atomicMax(&sMax[le * DIM + d], hi);
     }
-    atomicMax(&sMax[le], hi);
     const double pj = eg::pressure<DIM>(g, qj);
     if (!(qj[0] > 0.0)) atomicOr(status, EG_DEV_NEG_DENSITY);
     if (!(pj > 0.0)) atomicOr(status, EG_DEV_NEG_PRESSURE);
@@ -133,10 +150,15 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
     for (int c = 0; c < NV; ++c) sres[(size_t)t * NV + c] = 0.0;
   }
   __syncthreads();
-  const int exD = active ? exponent_above(sMax[le]) : 0;
-  if (active) {
+  int ex[DIM];  // n_jk[d] is in units of 2^(ex[d] + pair's exponent)
 #pragma unroll
-    for (int c = 0; c < D2; ++c) sD[c * rows + t] = dx[c] = to_limbs(dxd[c], exD);
+  for (int d = 0; d < DIM; ++d) {
+    const int e = active ? exponent_above(sMax[le * DIM + d]) : 0;
+    if (active) {
+#pragma unroll
+      for (int m = 0; m < DIM; ++m) sD[(d * DIM + m) * rows + t] = dx[d * DIM + m] = to_limbs(dxd[d * DIM + m], e);
+    }
+    ex[d] = e - 60;
   }
   // The logarithms are for pairs whose ratio of z1 or zp exceeds 1.065 (u above
   // 1e-3).  Nodes all within 3 % of the element's first have no such pair
@@ -167,7 +189,8 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
         qa[m] = sQa[(s * DIM + m) * Np + j];
         qb[m] = sQb[(s * DIM + m) * Np + j];
       }
-      double n[DIM];  // 2 S_x[j,k,:] times 2^(60 - exD - exQ)
+      const int eq = md.Qexp[s * Np + j];
+      double n[DIM];  // 2 S_x[j,k,:]
 #pragma unroll
       for (int d = 0; d < DIM; ++d) {
         long long hh = 0, x = 0;
@@ -178,7 +201,7 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
           x += (long long)a.h * qa[m].l + (long long)a.l * qa[m].h;
           x -= (long long)b.h * qb[m].l + (long long)b.l * qb[m].h;
         }
-        n[d] = (double)((hh << 2) + (x >> 28));
+        n[d] = scaled((hh << 2) + ((x + (1 << 27)) >> 28), ex[d] + eq);
       }
       const eg::IRNode<DIM> no{sN[0 * rows + o], sN[1 * rows + o], sN[2 * rows + o], sN[3 * rows + o],
                                sN[4 * rows + o], sN[5 * rows + o], sN[6 * rows + o]};
@@ -195,14 +218,8 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
     __syncthreads();
   }
   if (active) {
-    // value = n 2^(exD + exQ - 60)
-    const int k = exD + exQ - 60, k1 = k / 2;
-    const double f1 = pow2(k1), f2 = pow2(k - k1);
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      double* r = sres + (size_t)t * NV + c;
-      *r = (*r + acc[c]) * f1 * f2;
-    }
+    for (int c = 0; c < NV; ++c) sres[(size_t)t * NV + c] += acc[c];
   }
   __syncthreads();
   face_lift_smem<DIM>(md, fflux, sres, sL, sPerm, e0, nloc);
@@ -215,8 +232,8 @@ __global__ void k_split_element(DevMesh md, const double* __restrict__ q, const 
   split_element<DIM>(md, q, fflux, ep, status, epb);
 }
 
-// The pair loop takes 114 registers (84 on triangles), too many for a block of
-// more than 544 (736) threads to launch.  Wider blocks, which only an explicit
+// The pair loop takes 122 registers (88 on triangles), too many for a block of
+// more than 512 (736) threads to launch.  Wider blocks, which only an explicit
 // launch configuration or the autotuner asks for, run a build held to the
 // registers that MAXT threads leave.
 template <int DIM, int MAXT>
