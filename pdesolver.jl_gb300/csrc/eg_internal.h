@@ -51,6 +51,9 @@ struct TimerState;     // event pool (eg_timing.cu)
 struct eg_newton_ws;   // cached Newton work objects (eg_solvers.cu)
 struct eg_rk4_ws;      // cached RK4 work vectors and step graphs (eg_solvers.cu)
 
+// scale of a split-form pair or metric row with an entry that is not finite
+constexpr int EG_QEXP_NONFINITE = 1 << 20;
+
 struct eg_mesh {
   // sizes
   int dim, E, Np, Nf, S, F, I, B, nbc, norient, nv;

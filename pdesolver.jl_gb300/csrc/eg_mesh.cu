@@ -293,13 +293,18 @@ extern "C" int eg_mesh_create(const eg_mesh_desc* d, const eg_params* params, eg
     for (int j = 0; j < Np; ++j) {
       const int o = (j + s + 1) % Np;
       double qmax = 0.0;
-      for (int k = 0; k < 2 * dim; ++k) qmax = std::fmax(qmax, std::fabs(Qjo(k / 2, k % 2, j, o)));
-      const int ex = qmax > 0.0 && std::isfinite(qmax) ? std::ilogb(qmax) + 1 : 0;
+      bool finite = true;
+      for (int k = 0; k < 2 * dim; ++k) {
+        const double x = Qjo(k / 2, k % 2, j, o);
+        finite = finite && std::isfinite(x);
+        qmax = std::fmax(qmax, std::fabs(x));
+      }
+      const int ex = !finite ? EG_QEXP_NONFINITE : qmax > 0.0 ? std::ilogb(qmax) + 1 : 0;
       Qpair[(size_t)4 * H * dim * Np + (size_t)s * Np + j] = ex;
       for (int k = 0; k < dim; ++k)
         for (int side = 0; side < 2; ++side) {
           const double x = Qjo(k, side, j, o);
-          const long long v = std::isfinite(x) ? std::llrint(std::ldexp(x, 59 - ex)) : 0;
+          const long long v = finite ? std::llrint(std::ldexp(x, 59 - ex)) : 0;
           const long long h = (v + (1 << 29)) >> 30;
           int32_t* q = Qpair.data() + (((size_t)(side * H + s) * dim + k) * Np + j) * 2;
           q[0] = (int32_t)h;

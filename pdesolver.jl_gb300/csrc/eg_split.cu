@@ -53,11 +53,11 @@ struct Limbs {
   int h, l;
 };
 __device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-// smallest e with |x| < 2^e for the largest high word of |x| (normal range;
-// subnormals count as 2^-1022, infinities and NaN as 2^1024, zero as 1)
+// smallest e with |x| < 2^e for the largest high word of |x| (subnormals count
+// as 2^-1022, zero as 1, infinities and NaN as EG_QEXP_NONFINITE)
 __device__ __forceinline__ int exponent_above(int hi) {
-  const int b = (hi >> 20) & 0x7ff;
-  return hi == 0 ? 0 : (b < 1 ? 1 : b) - 1022;
+  const int b = hi >> 20;
+  return hi == 0 ? 0 : b == 0x7ff ? EG_QEXP_NONFINITE : (b < 1 ? 1 : b) - 1022;
 }
 __device__ __forceinline__ Limbs to_limbs(double x, int ex) {
   // two exact scalings: 59 - ex may exceed the exponent range of one
@@ -67,10 +67,11 @@ __device__ __forceinline__ Limbs to_limbs(double x, int ex) {
   return Limbs{h, (int)(v - ((long long)h << 30))};
 }
 // v 2^k: the exponent field takes k (v = 0 has none), or beyond its range three
-// products
+// products; NaN where a metric or Q entry is not finite
 __device__ __forceinline__ double scaled(long long v, int k) {
   const double x = (double)v;
   if (abs(k) <= 900) return v == 0 ? 0.0 : __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x));
+  if (k > EG_QEXP_NONFINITE / 2) return __longlong_as_double(0x7ff8000000000000LL);
   const int k3 = k / 3;
   return x * pow2(k3) * pow2(k3) * pow2(k - 2 * k3);
 }
