@@ -237,7 +237,7 @@ struct GmresShared {
   T scs[32], ssn[32], sg[33], syT[33];
   T sR[32 * 33];  // rotated Hessenberg columns: sR[j * (m+1) + k]
   double sRd[sizeof(T) == 4 ? 32 * 33 : 1];  // the same in FP64, for the back substitution
-  int s_done, s_its, s_jdone, s_conv, s_cycles, s_nreorth, s_reorth;
+  int s_done, s_its, s_jdone, s_conv, s_cycles, s_nreorth, s_err, s_reorth;
   T s_beta, s_g0, s_hn, s_inv, s_a1;
   double s_tol, s_bnorm;
 };
@@ -282,25 +282,29 @@ constexpr int kDirect = 32;
 
 // After a poll that failed: true when the wait is over without its word.  The
 // wait that runs out of polls raises flags[F_GAVE_UP], which every wait samples,
-// so all blocks leave.  A thread that gave up waits no more, its block returns
-// at the next barrier and publishes nothing that depends on the missing word:
-// every word that carries its tag is a good one.
+// so all blocks leave.  s_err is the block's own flag: its threads wait no more,
+// return after the next barrier and publish nothing that depends on the missing
+// word, so every word that carries its tag is a good one.  (A flag in shared
+// memory, and the rare part out of line: as a vote of the barrier and inlined,
+// spills cost the 24-unknown kernel 30 %.)
+__device__ __noinline__ bool give_up_now(volatile int* gave_up, bool out, volatile int* s_err) {
+  if (out) *gave_up = 1;
+  if (*gave_up) *s_err = 1;
+  return *s_err != 0;
+}
 template <typename T>
-__device__ __forceinline__ bool give_up(const CoopArgs<T>& a, int& polls) {
+__device__ __forceinline__ bool give_up(const CoopArgs<T>& a, int& polls, int* s_err) {
   ++polls;
-  if (polls > a.polls) {
-    atomicExch(a.flags + F_GAVE_UP, 1);
-    return true;
-  }
-  return (polls & 255) == 0 && *(volatile int*)(a.flags + F_GAVE_UP) != 0;
+  return ((polls & 255) == 0 || polls > a.polls) && give_up_now(a.flags + F_GAVE_UP, polls > a.polls, s_err);
 }
 
-// poll one word until it carries the tag; bad: given up
+// poll one word until it carries the tag
 template <typename T>
-__device__ __forceinline__ T word_wait(const CoopArgs<T>& a, const uint64_t* p, unsigned tag, bool& bad) {
-  T val = T(0);
+__device__ __forceinline__ T word_wait(const CoopArgs<T>& a, const uint64_t* p, unsigned tag, int* s_err) {
+  T val;
   int polls = 0;
-  while (!bad && !msg_get(p, tag, val)) bad = give_up(a, polls);
+  while (!msg_get(p, tag, val))
+    if (give_up(a, polls, s_err)) break;
   return val;
 }
 // publish this block's partial k of reduction `tag` (lane 0 of a warp)
@@ -309,27 +313,26 @@ __device__ __forceinline__ void part_put(const CoopArgs<T>& a, const BlockView<T
   if ((threadIdx.x & 31) == 0)
     msg_put(a.part + (size_t)(((tag & 1) * 33 + k) * v.nblk + v.b) * kWords<T>, val, tag);
 }
-// out[k] = sum over the blocks of partial k < cnt, the same bits in every
-// block; true in a thread that gave up
+// out[k] = sum over the blocks of partial k < cnt, the same bits in every block
 template <typename T>
-__device__ __forceinline__ bool part_sum(const CoopArgs<T>& a, const BlockView<T>& v, int cnt, T* out, unsigned tag) {
-  bool bad = false;
+__device__ __forceinline__ void part_sum(const CoopArgs<T>& a, const BlockView<T>& v, int cnt, T* out, unsigned tag,
+                                         int* s_err) {
   const int lane = threadIdx.x & 31, k = threadIdx.x >> 5;
   if (v.nblk <= kDirect) {
-    if (k >= cnt) return false;
+    if (k >= cnt) return;
     const uint64_t* p = a.part + (size_t)((tag & 1) * 33 + k) * v.nblk * kWords<T>;
     T acc = T(0);
-    for (int r = lane; r < v.nblk; r += 32) acc += word_wait(a, p + r * kWords<T>, tag, bad);
+    for (int r = lane; r < v.nblk; r += 32) acc += word_wait(a, p + r * kWords<T>, tag, s_err);
     acc = wsum(acc);
     if (lane == 0) out[k] = acc;
-    return bad;
+    return;
   }
   if (k < cnt && v.b == k * (v.nblk / 33)) {
     const uint64_t* p = a.part + (size_t)((tag & 1) * 33 + k) * v.nblk * kWords<T>;
     T acc = T(0);
     int polls = 0;
     constexpr int U = 5;
-    for (int b0 = lane; b0 < v.nblk && !bad; b0 += 32 * U) {
+    for (int b0 = lane; b0 < v.nblk; b0 += 32 * U) {
       T val[U];
       bool all;
       do {
@@ -339,18 +342,17 @@ __device__ __forceinline__ bool part_sum(const CoopArgs<T>& a, const BlockView<T
           val[u] = T(0);
           if (b0 + 32 * u < v.nblk) all &= msg_get(p + (size_t)(b0 + 32 * u) * kWords<T>, tag, val[u]);
         }
-        if (!all) bad = give_up(a, polls);
-      } while (!all && !bad);
+        if (!all && give_up(a, polls, s_err)) break;
+      } while (!all);
 #pragma unroll
       for (int u = 0; u < U; ++u) acc += val[u];
     }
-    const bool good = !__any_sync(0xffffffffu, bad);
     acc = wsum(acc);
-    if (lane == 0 && good) msg_put(a.tot + (size_t)((tag & 1) * 33 + k) * kLine, acc, tag);
+    __syncwarp();
+    if (lane == 0 && !*(volatile int*)s_err) msg_put(a.tot + (size_t)((tag & 1) * 33 + k) * kLine, acc, tag);
   }
   if (k == 31 && lane < cnt)
-    out[lane] = word_wait(a, a.tot + (size_t)((tag & 1) * 33 + lane) * kLine, tag, bad);
-  return bad;
+    out[lane] = word_wait(a, a.tot + (size_t)((tag & 1) * 33 + lane) * kLine, tag, s_err);
 }
 
 // partial dots of the block's rows against x: warp k < cnt takes V[k] (plus
@@ -614,11 +616,10 @@ __device__ __forceinline__ void build_push_operator(const CoopArgs<T>& a, const 
 
 // Sum of the pushed products that land on row (node j, variable av) of own
 // element le, in face order: one term per simplex face whose stencil holds the
-// node and that couples to a neighbour.  Polls until all of them carry `tag`;
-// bad: given up.
+// node and that couples to a neighbour.  Polls until all of them carry `tag`.
 template <int DIM, typename T>
 __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v, const int* sSpos, int le, int j,
-                                    int av, unsigned tag, bool& bad) {
+                                    int av, unsigned tag, int* s_err) {
   constexpr int NV = DIM + 2, FF = DIM + 1;
   const uint64_t* p[FF];
 #pragma unroll
@@ -637,8 +638,8 @@ __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v,
       val[f] = T(0);
       if (p[f]) all &= msg_get(p[f], tag, val[f]);
     }
-    if (!all) bad = give_up(a, polls);
-  } while (!all && !bad);
+    if (!all && give_up(a, polls, s_err)) break;
+  } while (!all);
   T acc = T(0);
 #pragma unroll
   for (int f = 0; f < FF; ++f) acc += val[f];
@@ -786,7 +787,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
   for (int k = tid; k < a.F * a.S; k += NT) sm.sPerm[k] = a.md.perm[k];
   for (int k = tid; k < a.F * Np; k += NT) sm.sSpos[k] = a.spos[k];
   if (tid == 0) {
-    sm.s_its = sm.s_cycles = sm.s_nreorth = 0;
+    sm.s_its = sm.s_cycles = sm.s_nreorth = sm.s_err = 0;
     sm.s_conv = 0;
     // nodes on some face stencil first (face-diagonal operators: all nodes)
     int q = 0;
@@ -823,7 +824,9 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       const T s = wsum(sm.sR[32 * wq + lane]);
       part_put(a, v, wq, s, rt);
     }
-    if (__syncthreads_or(part_sum(a, v, 2, sm.sh1, rt))) return;
+    part_sum(a, v, 2, sm.sh1, rt, &sm.s_err);
+    __syncthreads();
+    if (sm.s_err) return;
     if (tid == 0) {
       sm.s_bnorm = sqrt(double(sm.sh1[0]));
       sm.s_tol = fmax(a.scal[S_RELTOL] * sm.s_bnorm, a.scal[S_ABSTOL]);
@@ -833,24 +836,24 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
   __syncthreads();
   for (;;) {
     // ---- r = b - J x (natural rows, in a.w); the pushed products cross blocks
-    bool bad = false;
     if (xzero) {
       for (int t = tid; t < nat; t += NT) a.w[r0 + t] = a.bvec[r0 + t];
     } else {
       ++pt;
       couple_push<DIM, T>(a, v, a.x + r0, 0, v.nel, sm.sPerm, pt, pol);
-      for (int t = tid; t < nat && !bad; t += NT) {
+      for (int t = tid; t < nat; t += NT) {
         const int le = t / n, r = t - le * n;
         const int e = v.e0 + le;
         const T* A = a.diag + (size_t)e * n * n;
         const T* xe = a.x + (size_t)e * n;
         const T d = a.trans ? block_col<T>(A, xe, r, n) : block_row<NB, T>(A, xe, r, n);
         const int j = r / NV;
-        a.w[r0 + t] = a.bvec[r0 + t] - (d + gather<DIM, T>(a, v, sm.sSpos, le, j, r - j * NV, pt, bad));
+        a.w[r0 + t] = a.bvec[r0 + t] - (d + gather<DIM, T>(a, v, sm.sSpos, le, j, r - j * NV, pt, &sm.s_err));
       }
     }
     xzero = false;
-    if (__syncthreads_or(bad)) return;
+    __syncthreads();
+    if (sm.s_err) return;
     // |r|^2 of the stencil rows and of the interior rows
     {
       const int lane = tid & 31, wq = tid >> 5;
@@ -874,7 +877,9 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
         const T s = wsum(sm.sR[32 * wq + lane]);
         part_put(a, v, wq, s, rt);
       }
-      if (__syncthreads_or(part_sum(a, v, 2, sm.sh1, rt))) return;
+      part_sum(a, v, 2, sm.sh1, rt, &sm.s_err);
+      __syncthreads();
+      if (sm.s_err) return;
     }
     if (tid == 0) {
       const T b2 = sm.sh1[0] + sm.sh1[1];
@@ -936,17 +941,20 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       __syncthreads();
       if (sm.s_done) break;
       // (2) w = K v_j: the pushed products of the faces holding the row's node
-      for (int t = tid; t < nrow && !bad; t += NT) {
+      for (int t = tid; t < nrow; t += NT) {
         const int le = t / nbd, q = t - le * nbd;
         const int jn = q / NV;
-        v.sw[t] = gather<DIM, T>(a, v, sm.sSpos, le, sm.sOrd[jn], q - jn * NV, pt, bad);
+        v.sw[t] = gather<DIM, T>(a, v, sm.sSpos, le, sm.sOrd[jn], q - jn * NV, pt, &sm.s_err);
       }
       if (tid < v.nrowp - nrow) v.sw[nrow + tid] = T(0);
-      if (__syncthreads_or(bad)) return;
+      __syncthreads();
+      if (sm.s_err) return;
       // (3) first pass: h1 = V^T w and w.w in one reduction
       ++rt;
       dots_put<T>(a, v, v.sw, j + 1, T(0), T(0), sm.sal, rt);
-      if (__syncthreads_or(part_sum(a, v, j + 2, sm.sh1, rt))) return;
+      part_sum(a, v, j + 2, sm.sh1, rt, &sm.s_err);
+      __syncthreads();
+      if (sm.s_err) return;
       if (tid < 32) {
         T hh, a1;
         column_sums(sm.sh1, sm.sal, j, hh, a1);
@@ -972,7 +980,9 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
         __syncthreads();
         ++rt;
         dots_put<T>(a, v, v.sw, j + 1, sm.s_a1, sm.s_g0, sm.sal, rt);
-        if (__syncthreads_or(part_sum(a, v, j + 2, sm.sh2, rt))) return;
+        part_sum(a, v, j + 2, sm.sh2, rt, &sm.s_err);
+        __syncthreads();
+        if (sm.s_err) return;
         if (tid < 32) {
           T hh, a2;
           column_sums(sm.sh2, sm.sal, j, hh, a2);
