@@ -236,7 +236,10 @@ struct GmresShared {
   T sal[33];      // interior part of v_k = sal[k] * vint
   T scs[32], ssn[32], sg[33], syT[33];
   T sR[32 * 33];  // rotated Hessenberg columns: sR[j * (m+1) + k]
-  double sRd[sizeof(T) == 4 ? 32 * 33 : 1];  // the same in FP64, for the back substitution
+  // the same in FP64: columns for the back substitution; transposed FP32 solves
+  // rotate in FP64 throughout
+  double sRd[sizeof(T) == 4 ? 32 * 33 : 1];
+  double dcs[sizeof(T) == 4 ? 32 : 1], dsn[sizeof(T) == 4 ? 32 : 1], dg[sizeof(T) == 4 ? 33 : 1];
   int s_done, s_its, s_jdone, s_conv, s_cycles, s_nreorth, s_err, s_reorth;
   T s_beta, s_g0, s_hn, s_inv, s_a1;
   double s_tol, s_bnorm;
@@ -286,7 +289,7 @@ constexpr int kDirect = 32;
 // return after the next barrier and publish nothing that depends on the missing
 // word, so every word that carries its tag is a good one.  (A flag in shared
 // memory, and the rare part out of line: as a vote of the barrier and inlined,
-// spills cost the 24-unknown kernel 30 %.)
+// spills made 8,192 triangles Omega p=2 12 % slower.)
 __device__ __noinline__ bool give_up_now(volatile int* gave_up, bool out, volatile int* s_err) {
   if (out) *gave_up = 1;
   if (*gave_up) *s_err = 1;
@@ -646,57 +649,76 @@ __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v,
   return acc;
 }
 
-// Hessenberg column j and its Givens rotation in T by one warp (identical in
-// every block); h = h1 (+ h2 after a second pass), hn = |w'|.  The j earlier
+// Hessenberg column j and its Givens rotation in R (T, or FP64 for a transposed
+// FP32 solve) by one warp (identical in every block), to the rotations rcs, rsn,
+// the right-hand side rg and the columns rR; h = h1 (+ h2 after a second pass),
+// hn = |w'|.  The j earlier
 // rotations act on the column as the affine recurrence t_0 = h_0, t_{k+1} =
 // -sn_k t_k + cs_k h_{k+1} (row k becomes cs_k t_k + sn_k h_{k+1}), evaluated
 // by a scan over the lanes instead of j dependent steps (the serial form took
 // longer than the apply that it runs beside on small systems).
-template <typename T>
-__device__ __forceinline__ void givens(GmresShared<T>& sm, int j, int M1, int itermax) {
+template <typename R, typename T>
+__device__ __forceinline__ void givens(GmresShared<T>& sm, int j, int M1, int itermax, R* rcs, R* rsn, R* rg, R* rR) {
   const int lane = threadIdx.x & 31;
   const bool reorth = sm.s_reorth != 0;
-  const T hn = sm.s_hn;
+  const R hn = R(sm.s_hn);
   // column j of H_K + I, the Hessenberg matrix of I + K: lane k holds h_k
-  T h = lane <= j ? sm.sh1[lane] : T(0);
-  if (reorth && lane <= j) h += sm.sh2[lane];
-  if (lane == j) h += T(1);
-  const T h0 = __shfl_sync(0xffffffffu, h, 0);
-  const T hup = __shfl_down_sync(0xffffffffu, h, 1);  // h_{k+1}
-  const T cs = lane < j ? sm.scs[lane] : T(1), sn = lane < j ? sm.ssn[lane] : T(0);
-  T A = lane < j ? -sn : T(1), B = lane < j ? cs * hup : T(0);
+  R h = lane <= j ? R(sm.sh1[lane]) : R(0);
+  if (reorth && lane <= j) h += R(sm.sh2[lane]);
+  if (lane == j) h += R(1);
+  const R h0 = __shfl_sync(0xffffffffu, h, 0);
+  const R hup = __shfl_down_sync(0xffffffffu, h, 1);  // h_{k+1}
+  const R cs = lane < j ? rcs[lane] : R(1), sn = lane < j ? rsn[lane] : R(0);
+  R A = lane < j ? -sn : R(1), B = lane < j ? cs * hup : R(0);
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const T Al = __shfl_up_sync(0xffffffffu, A, o), Bl = __shfl_up_sync(0xffffffffu, B, o);
+    const R Al = __shfl_up_sync(0xffffffffu, A, o), Bl = __shfl_up_sync(0xffffffffu, B, o);
     if (lane >= o) {
       B = A * Bl + B;
       A = A * Al;
     }
   }
-  const T tn = A * h0 + B;  // t_{k+1}
-  T t = __shfl_up_sync(0xffffffffu, tn, 1);
+  const R tn = A * h0 + B;  // t_{k+1}
+  R t = __shfl_up_sync(0xffffffffu, tn, 1);
   if (lane == 0) t = h0;  // t_k
-  if (lane < j) sm.sR[j * M1 + lane] = cs * t + sn * hup;
+  if (lane < j) rR[j * M1 + lane] = cs * t + sn * hup;
   t = __shfl_sync(0xffffffffu, t, j);
   if (lane == 0) {
-    const T den = hypot(t, hn);
+    R den, id;
+    if constexpr (sizeof(R) > sizeof(T)) {  // squares of FP32 values stay in range
+      const R s2 = t * t + hn * hn;
+      id = rsqrt(s2);
+      den = s2 > R(0) ? s2 * id : s2;
+    } else {
+      den = hypot(t, hn);
+      id = R(1) / den;
+    }
     sm.s_its += 1;
-    if (!(den > T(0)) || !isfinite(den)) {
+    if (!(den > R(0)) || !isfinite(den)) {
       sm.s_done = 1;  // breakdown: keep the j columns built so far
     } else {
-      const T id = T(1) / den;
-      const T c = t * id, s = hn * id;
-      sm.scs[j] = c;
-      sm.ssn[j] = s;
-      sm.sR[j * M1 + j] = den;
-      const T g = sm.sg[j];
-      sm.sg[j + 1] = -s * g;
-      sm.sg[j] = c * g;
+      const R c = t * id, s = hn * id;
+      rcs[j] = c;
+      rsn[j] = s;
+      rR[j * M1 + j] = den;
+      const R g = rg[j];
+      rg[j + 1] = -s * g;
+      rg[j] = c * g;
       sm.s_jdone = j + 1;
       const double resid = fabs(double(s * g));
-      if (resid <= sm.s_tol || hn == T(0) || sm.s_its >= itermax) sm.s_done = 1;
+      if (resid <= sm.s_tol || hn == R(0) || sm.s_its >= itermax) sm.s_done = 1;
     }
   }
+}
+template <typename T>
+__device__ __forceinline__ void givens(const CoopArgs<T>& a, GmresShared<T>& sm, int j, int M1) {
+  if constexpr (sizeof(T) == 4) {
+    if (a.trans) {
+      givens<double>(sm, j, M1, a.flags[F_ITERMAX], sm.dcs, sm.dsn, sm.dg, sm.sRd);
+      return;
+    }
+  }
+  givens<T>(sm, j, M1, a.flags[F_ITERMAX], sm.scs, sm.ssn, sm.sg, sm.sR);
 }
 
 // After a reduction, by one warp: |h|^2 and the interior coefficient sum h_k
@@ -894,6 +916,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       sm.s_jdone = 0;
       sm.sg[0] = beta;
       for (int k = 1; k <= m; ++k) sm.sg[k] = T(0);
+      if (sizeof(T) == 4 && a.trans) sm.dg[0] = double(beta);
     }
     __syncthreads();
     if (sm.s_done) break;
@@ -935,7 +958,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       // (1) push K v_j; meanwhile one warp finishes column j - 1 (Hessenberg,
       //     rotation, convergence)
       ++pt;
-      if (tid < 32 && j > 0) givens(sm, j - 1, M1, a.flags[F_ITERMAX]);
+      if (tid < 32 && j > 0) givens(a, sm, j - 1, M1);
       apply_push<DIM, NB, T>(a, v, a.ws ? v.cur : basis(a, v, j), sm.sal[j], sm.sPerm, pt,
                              a.md.sparse_face ? 0 : 32, pol);
       __syncthreads();
@@ -1002,7 +1025,7 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
       sub_scale<T>(a, v, hl, j + 1, v.sw, sm.s_inv, vn, a.ws ? v.cur : vn);
       __syncthreads();
       if (++j == m) {
-        if (tid < 32) givens(sm, m - 1, M1, a.flags[F_ITERMAX]);
+        if (tid < 32) givens(a, sm, m - 1, M1);
         __syncthreads();
         break;
       }
@@ -1010,18 +1033,21 @@ __device__ void gmres_body(const CoopArgs<T>& a, const int b, const int nblk, Gm
     // ---- y = R^-1 g (FP64 back substitution by warp 0), x += D^-1 V y
     const int nn = sm.s_jdone;
     if constexpr (sizeof(T) == 4) {
-      for (int t = tid; t < nn * M1; t += NT) sm.sRd[t] = double(sm.sR[t]);
-      __syncthreads();
+      if (!a.trans) {
+        for (int t = tid; t < nn * M1; t += NT) sm.sRd[t] = double(sm.sR[t]);
+        if (tid < nn) sm.dg[tid] = double(sm.sg[tid]);
+        __syncthreads();
+      }
     }
     if (tid < 32) {
       // lane i holds g_i and 1 / R_ii; y_k is broadcast from lane k.  The
       // chain per step is one multiply, the broadcast and one FMA: FP64
       // conversions and shared-memory stores in it cost more than the step
       const int lane = tid;
-      const double* R;
-      if constexpr (sizeof(T) == 4) R = sm.sRd;
-      else R = sm.sR;
-      double g = lane < nn ? double(sm.sg[lane]) : 0.0, y = 0.0;
+      const double *R, *rg;
+      if constexpr (sizeof(T) == 4) R = sm.sRd, rg = sm.dg;
+      else R = sm.sR, rg = sm.sg;
+      double g = lane < nn ? rg[lane] : 0.0, y = 0.0;
       const double di = lane < nn ? 1.0 / R[lane * M1 + lane] : 0.0;
 #pragma unroll 2
       for (int k = nn - 1; k >= 0; --k) {
