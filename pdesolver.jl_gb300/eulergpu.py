@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import threading
 
 import numpy as np
 
@@ -185,6 +186,31 @@ def set_gmres_batching(enable=True, window_us=50.0):
     check(library().eg_set_gmres_batching(int(bool(enable)), float(window_us)))
 
 
+class _Native:
+    """A library object and the ones that it was made from: it is destroyed when
+    it and everything made from it has been closed, so that children go first
+    in whatever order Python finalises the objects of a reference cycle (an
+    exception's frames make one)."""
+
+    _lock = threading.RLock()   # a finaliser may run inside another's count
+
+    def __init__(self, handle, destroy, parents=()):
+        self.handle, self.destroy, self.parents = handle, destroy, parents
+        self.users = 1
+        with self._lock:
+            for p in parents:
+                p.users += 1
+
+    def drop(self):
+        with self._lock:
+            self.users -= 1
+            last = self.users == 0
+        if last:
+            self.destroy(self.handle)
+            for p in self.parents:
+                p.drop()
+
+
 class GPUMesh:
     """Owner of one eg_mesh (device copy of mesh + operator + parameters)."""
 
@@ -197,6 +223,7 @@ class GPUMesh:
         h = C.c_void_p()
         check(self.lib.eg_mesh_create(C.byref(self.desc.desc), C.byref(self.params), C.byref(h)))
         self.handle = h
+        self.native = _Native(h, self.lib.eg_mesh_destroy)
         self.ndof = int(self.lib.eg_mesh_num_dof(h))
 
     def set_params(self, opts: dict):
@@ -230,8 +257,8 @@ class GPUMesh:
 
     def close(self):
         if getattr(self, "handle", None):
-            self.lib.eg_mesh_destroy(self.handle)
             self.handle = None
+            self.native.drop()
 
     def __del__(self):
         try:
@@ -473,6 +500,7 @@ class LinearOperator:
         h = C.c_void_p()
         check(self.lib.eg_lo_create(gmesh.handle, precision, C.byref(h)))
         self.handle = h
+        self.native = _Native(h, self.lib.eg_lo_destroy, (gmesh.native,))
         op = gmesh.mesh.sbp
         self.n = op.numnodes * gmesh.mesh.numDofPerNode
         self.nb = op.stencilsize * gmesh.mesh.numDofPerNode
@@ -518,8 +546,8 @@ class LinearOperator:
 
     def close(self):
         if getattr(self, "handle", None):
-            self.lib.eg_lo_destroy(self.handle)
             self.handle = None
+            self.native.drop()
 
     def __del__(self):
         try:
@@ -537,6 +565,7 @@ class BlockJacobiPC:
         h = C.c_void_p()
         check(self.lib.eg_pc_create(lo.handle, C.byref(h)))
         self.handle = h
+        self.native = _Native(h, self.lib.eg_pc_destroy, (lo.native,))
 
     def calc(self):
         check(self.lib.eg_pc_calc(self.handle))
@@ -566,8 +595,8 @@ class BlockJacobiPC:
 
     def close(self):
         if getattr(self, "handle", None):
-            self.lib.eg_pc_destroy(self.handle)
             self.handle = None
+            self.native.drop()
 
     def __del__(self):
         try:
@@ -585,6 +614,7 @@ class LinearSolver:
         h = C.c_void_p()
         check(self.lib.eg_ls_create(lo.handle, pc.handle, restart, C.byref(h)))
         self.handle = h
+        self.native = _Native(h, self.lib.eg_ls_destroy, (pc.native, lo.native))
         self.restart = restart
         self.reltol, self.abstol, self.itermax = -1.0, -1.0, -1
 
@@ -631,8 +661,8 @@ class LinearSolver:
 
     def close(self):
         if getattr(self, "handle", None):
-            self.lib.eg_ls_destroy(self.handle)
             self.handle = None
+            self.native.drop()
 
     def __del__(self):
         try:
