@@ -418,7 +418,8 @@ typedef struct {
 
 typedef struct {
   eg_launch_config config;
-  double ms;                 /* mean element-kernel time of the candidate       */
+  double ms;                 /* mean time of the candidate: element kernel, or  */
+                             /* whole residual (see eg_autotune)                */
 } eg_tune_entry;
 
 int eg_set_launch_config(eg_mesh* mesh, const eg_launch_config* config);
@@ -426,7 +427,10 @@ int eg_get_launch_config(eg_mesh* mesh, eg_launch_config* config);
 /* Autotuner: times every admissible configuration (elements per CTA 1, 2,
    4, ... up to 1024 threads, times CUDA-core / tensor-core contraction) on
    the state q_dev (device, [E][Np][nv]) over `reps` launches each, with CUDA
-   events on the mesh stream, and keeps the fastest on the mesh.  Up to
+   events on the mesh stream, and keeps the fastest on the mesh.  On a mesh
+   whose built-in configuration is the one-launch residual, that
+   configuration (0, 0) is a candidate too, and every candidate is timed as a
+   whole residual (face fluxes and element kernel).  Up to
    max_entries timings go to `table` (n_entries set to their count).
    Synchronises the mesh stream; not allowed during stream capture. */
 int eg_autotune(eg_mesh* mesh, const double* q_dev, int32_t reps, eg_tune_entry* table,

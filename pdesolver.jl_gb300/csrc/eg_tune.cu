@@ -8,7 +8,9 @@
 // whether the volume contraction Q^T F runs on CUDA cores or on the FP64
 // tensor cores (mma.sync m8n8k4).  eg_autotune times every admissible
 // candidate on the caller's state with CUDA events on the mesh stream and
-// keeps the fastest.  The reference has no counterpart (its loops are plain
+// keeps the fastest.  On a mesh small enough for the one-launch residual
+// (eg_small.cu) the built-in configuration is a candidate, and every candidate
+// is timed as a whole residual, since that launch takes the face fluxes too.  The reference has no counterpart (its loops are plain
 // Julia); the result changes only the launch shape and, for the tensor-core
 // contraction, the order of the FP64 sums (results agree with the CUDA-core
 // path to round-off).
@@ -74,6 +76,14 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
   m->elem_epb = 0;
   const int builtin = eg_elements_per_cta(m);
   m->elem_epb = own_epb;
+  eg_launch_config own;
+  std::memset(&own, 0, sizeof(own));
+  eg_mesh own_mesh = *m;
+  own_mesh.elem_epb = 0;
+  own_mesh.vol_mma = 0;
+  const bool one_launch =
+      eg_small_usable(&own_mesh, q_dev, Epilogue{0, 0.0, m->Minv, nullptr, nullptr, m->res_dev});
+  if (one_launch) cand.push_back(own);
   std::vector<int> sizes;
   for (int epb = 1; epb <= 128; epb *= 2) {
     if (builtin > epb / 2 && builtin < epb) sizes.push_back(builtin);
@@ -101,7 +111,9 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
   if (timers) eg_set_timing(m, 0);
   double* res = m->res_dev;
   // face fluxes of q once (an explicit configuration keeps to the two
-  // kernels); every candidate then reads the same m->fflux
+  // kernels); every candidate then reads the same m->fflux, unless it is timed
+  // as a whole residual
+  auto run = [&]() { return one_launch ? eg_launch_residual(m, q_dev, res) : eg_launch_element(m, q_dev, res); };
   m->elem_epb = builtin;
   m->vol_mma = 0;
   int st = eg_launch_residual(m, q_dev, res);
@@ -117,11 +129,11 @@ extern "C" int eg_autotune(eg_mesh* m, const double* q_dev, int32_t reps, eg_tun
   for (size_t k = 0; k < cand.size() && st == EG_OK; ++k) {
     m->elem_epb = cand[k].elements_per_cta;
     m->vol_mma = cand[k].volume_mma;
-    st = eg_launch_element(m, q_dev, res);  // warm-up (instruction cache, attributes)
+    st = run();  // warm-up (instruction cache, attributes)
     if (st != EG_OK) break;
     if (cudaGetLastError() != cudaSuccess) continue;  // this shape does not launch: no time to compare
     cudaEventRecord(ev0, m->stream);
-    for (int r = 0; r < reps && st == EG_OK; ++r) st = eg_launch_element(m, q_dev, res);
+    for (int r = 0; r < reps && st == EG_OK; ++r) st = run();
     cudaEventRecord(ev1, m->stream);
     cudaError_t e = cudaEventSynchronize(ev1);
     if (e != cudaSuccess) {
