@@ -94,6 +94,7 @@ struct eg_mesh {
   double* red;      // reduction scratch
   unsigned int* h_status; // pinned host mirror, and a word eg_eval_residual's kernels write
   bool status_clear;      // the device word is known to be zero
+  bool status_replays;    // a caller's graph holds kernels that set it: never known
   double* h_red;          // pinned host scalar
   cudaStream_t own_stream;  // the library's stream (stream may be a caller's)
   TimerState* timer;        // phase timers (null until enabled)
@@ -138,5 +139,7 @@ int eg_launch_element(eg_mesh* m, const double* q, double* res);
 // dynamic shared memory; EG_ERR_INVALID if the configuration does not fit
 int eg_element_shape(const eg_mesh* m, int epb, int mma, int* threads, size_t* smem);
 int eg_check_status(eg_mesh* m);
+// before an asynchronous entry point's kernels that may set the status word
+void eg_status_async(eg_mesh* m);
 // phase timers enabled (they take CUDA events from a growing pool)
 bool eg_timing_on(const eg_mesh* m);

@@ -698,7 +698,7 @@ extern "C" int eg_pc_calc(eg_pc* pc) {
     eg_set_error("eg_pc_calc: element block of %d unknowns exceeds shared memory", n);
     return EG_ERR_UNSUPPORTED;
   }
-  m->status_clear = false;
+  eg_status_async(m);
   eg_phase_begin(m, EG_PHASE_OTHER);
   const int st = eg_block_inverse(m, pc->lo->prec, pc->lo->diag, pc->inv, n);
   eg_phase_end(m, EG_PHASE_OTHER, 1);

@@ -543,6 +543,18 @@ int eg_check_status(eg_mesh* m) {
   return EG_OK;
 }
 
+void eg_status_async(eg_mesh* m) {
+  m->status_clear = false;
+  if (m->status_replays || m->capturing) return;
+  // launches captured by the caller run again with every replay
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(m->stream, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    m->status_replays = true;
+  }
+  if (cs != cudaStreamCaptureStatusNone) m->status_replays = true;
+}
+
 extern "C" int eg_eval_residual(eg_mesh* m, const double* q, double* res, double t, int32_t mem) {
   (void)t;  // the implemented boundary states are time-independent
   if (!m || !q || !res) {
@@ -561,9 +573,10 @@ extern "C" int eg_eval_residual(eg_mesh* m, const double* q, double* res, double
   // (h_status[1], which only this call uses; touched only when something is
   // wrong): no memset and no copy between the caller and a small residual.
   // This call ends synchronised, so nothing of an earlier one is in flight.
-  // The device word is cleared when other work may have set it, and takes the
-  // flags of an unphysical state, as if the kernels had written it.
-  if (!m->status_clear) EG_CUDA(cudaMemsetAsync(m->status, 0, sizeof(unsigned int), m->stream));
+  // The device word is cleared when other work may have set it (a replay of a
+  // caller's graph may at any time), and takes the flags of an unphysical
+  // state, as if the kernels had written it.
+  if (!m->status_clear || m->status_replays) EG_CUDA(cudaMemsetAsync(m->status, 0, sizeof(unsigned int), m->stream));
   unsigned int* const dev_status = m->status;
   volatile unsigned int* word = m->h_status + 1;
   *word = 0;

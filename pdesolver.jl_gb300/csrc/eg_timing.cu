@@ -152,6 +152,7 @@ extern "C" int eg_eval_residual_async(eg_mesh* m, const double* q, double* res) 
     eg_set_error("eg_eval_residual_async: NULL argument");
     return EG_ERR_INVALID;
   }
+  eg_status_async(m);
   int st = eg_launch_residual(m, q, res);
   if (st != EG_OK) return st;
   EG_CUDA(cudaGetLastError());
