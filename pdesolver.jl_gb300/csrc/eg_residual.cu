@@ -583,15 +583,14 @@ extern "C" int eg_eval_residual(eg_mesh* m, const double* q, double* res, double
   m->status = m->h_status + 1;
   int st = eg_launch_residual(m, qd, rd);
   m->status = dev_status;
-  m->status_clear = true;
   if (st != EG_OK) return st;
   EG_CUDA(cudaGetLastError());
   if (mem == EG_MEM_HOST)
     EG_CUDA(cudaMemcpyAsync(res, rd, bytes, cudaMemcpyDeviceToHost, m->stream));
   EG_CUDA(cudaStreamSynchronize(m->stream));
   *m->h_status = *word;
+  m->status_clear = !*word;
   if (*word) {
-    m->status_clear = false;
     EG_CUDA(cudaMemcpyAsync(m->status, m->h_status, sizeof(unsigned int), cudaMemcpyHostToDevice, m->stream));
   }
   return eg_check_status(m);
