@@ -445,8 +445,8 @@ int eg_newton_release(eg_mesh* mesh);
 /* rk4 (reference src/NonlinearSolvers/rk4.jl:144-336, 404-456): classical
    4-stage RK4 on dq/dt = M^-1 R(q) with step h for round(t_max/h) steps
    (fewer if itermax > 0 is reached, or if res_tol > 0 and the stage-1 norm
-   drops below it).  The first call on a mesh allocates six state-sized work
-   vectors (48 bytes per unknown) that the mesh keeps (eg_newton_release or
+   drops below it).  The first call on a mesh allocates four state-sized work
+   vectors (32 bytes per unknown) that the mesh keeps (eg_newton_release or
    destroy frees them).  With the phase timers off and a mesh stream that can
    be captured (not the legacy default stream), each time step is replayed as
    a CUDA graph captured on first use for this h (one graph per step; with
@@ -466,7 +466,7 @@ int eg_rk4(eg_mesh* mesh, double* q, double h, double t_max, int32_t itermax, do
    holds most of the HBM cannot count on a mid-run cudaMalloc, and cudaFree
    synchronises the whole device).  Same arguments, kernels and results as
    eg_rk4, for meshes of at most EG_RK4_STATIC_MAX_DOF unknowns (larger ones:
-   EG_ERR_INVALID); the work vectors live in one static 24 MiB device array
+   EG_ERR_INVALID); the work vectors live in one static 16 MiB device array
    per device.  The first call on a device resolves that array's address with
    the device current and should come before any stream capture (the address
    is resolved again if the device's context has changed, e.g. after

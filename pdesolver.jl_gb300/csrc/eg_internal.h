@@ -117,7 +117,7 @@ void eg_rk4_ws_free(eg_mesh* m);
 // stream belongs to it; EG_ERR_INVALID (with a message naming `who`) otherwise
 int eg_check_device(const eg_mesh* m, const char* who);
 // The RK4 step loop of eg_rk4 (reference rk4.jl:201-330) on the device
-// buffers buf[6][ndof] (x first, q last), with x = the start state already in
+// buffers buf[4][ndof] (x first, q last), with x = the start state already in
 // place and the status word cleared; the result is in q.  use_graphs:
 // replay captured CUDA graphs of the step (the mesh keeps them) where the
 // stream can be captured.  On return the stream has no work of the loop left

@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(NT) k_small_residual(DevMesh md, const double*
       } else if (!interior || md.face_flux == EG_FLUX_ROE) {
         eg::roe_flux<DIM>(g, qL, qR, nrm, fl);
       } else {
-        const auto nL = eg::ir_node<DIM, false>(g, qL);
-        const auto nR = eg::ir_node<DIM, false>(g, qR);
+        const auto nL = eg::ir_node<DIM>(g, qL);
+        const auto nR = eg::ir_node<DIM>(g, qR);
         const auto av = eg::ir_average_pre<DIM, false>(g, nL, nR);
         eg::ir_dir<DIM>(av, nrm, fl);
       }

@@ -603,13 +603,13 @@ extern "C" int eg_newton_solve(eg_mesh* m, double* q, int32_t mem, const eg_newt
   return st;
 }
 
-// RK4 work objects a mesh keeps between eg_rk4 calls: the six state-sized
+// RK4 work objects a mesh keeps between eg_rk4 calls: the four state-sized
 // vectors of the step loop, and CUDA graphs of one step (whole step; stage 1
 // with the norm read-back; stages 2-4), captured on first use and bound to
 // the vectors, the step size and the launch configuration they were taken
 // with.
 struct eg_rk4_ws {
-  double* buf = nullptr;  // [6][N]: x, acc, stage state, unused, unused, q
+  double* buf = nullptr;  // [4][N]: x, acc, stage state, q
   bool tried = false;     // capture attempted for `key`
   bool have = false;      // graphs valid for `key`
   struct {
@@ -638,7 +638,7 @@ void rk4_graphs_free(eg_rk4_ws* w) {
 // and no pass over the state of its own.
 int rk4_stage1(eg_mesh* m, double* buf, double h, bool with_norm) {
   const int64_t N = m->ndof;
-  double *x = buf, *acc = buf + N, *q = buf + 5 * N;
+  double *x = buf, *acc = buf + N, *q = buf + 3 * N;
   const int st = eg_launch_stage(m, x, Epilogue{1, h / 2, m->Minv, x, acc, q});
   if (st != EG_OK) return st;
   if (with_norm) {
@@ -652,7 +652,7 @@ int rk4_stage1(eg_mesh* m, double* buf, double h, bool with_norm) {
 // stages 2, 3, 4 and the update of x
 int rk4_rest(eg_mesh* m, double* buf, double h) {
   const int64_t N = m->ndof;
-  double *x = buf, *acc = buf + N, *p = buf + 2 * N, *q = buf + 5 * N;
+  double *x = buf, *acc = buf + N, *p = buf + 2 * N, *q = buf + 3 * N;
   int st = eg_launch_stage(m, q, Epilogue{2, h / 2, m->Minv, x, acc, p});
   if (st == EG_OK) st = eg_launch_stage(m, p, Epilogue{2, h, m->Minv, x, acc, q});
   if (st == EG_OK) st = eg_launch_stage(m, q, Epilogue{3, h / 6, m->Minv, x, acc, x});
@@ -691,7 +691,7 @@ bool rk4_graphs(eg_mesh* m, eg_rk4_ws* w, double h) {
 int rk4_ws(eg_mesh* m, eg_rk4_ws** out) {
   if (!m->rws) {
     eg_rk4_ws* w = new eg_rk4_ws();
-    cudaError_t ce = cudaMalloc((void**)&w->buf, 6 * 8 * (size_t)m->ndof);
+    cudaError_t ce = cudaMalloc((void**)&w->buf, 4 * 8 * (size_t)m->ndof);
     if (ce != cudaSuccess) {
       delete w;
       return eg_cuda_fail(ce, "eg_rk4");
@@ -779,7 +779,7 @@ int eg_rk4_loop(eg_mesh* m, double* buf, double h, double t_max, int itermax, do
   }
   t += h;
   if (st == EG_OK && whole) {
-    const cudaError_t ce = cudaMemcpyAsync(buf + 5 * m->ndof, buf, 8 * (size_t)m->ndof, cudaMemcpyDeviceToDevice,
+    const cudaError_t ce = cudaMemcpyAsync(buf + 3 * m->ndof, buf, 8 * (size_t)m->ndof, cudaMemcpyDeviceToDevice,
                                            m->stream);
     if (ce != cudaSuccess) st = eg_cuda_fail(ce, "eg_rk4");
   }
@@ -806,9 +806,9 @@ extern "C" int eg_rk4(eg_mesh* m, double* q, double h, double t_max, int32_t ite
   if ((st = rk4_ws(m, &w)) != EG_OK) return st;
   const int64_t N = m->ndof;
   double* buf = w->buf;
-  double* qd = buf + 5 * N;
+  double* qd = buf + 3 * N;
   // the loop iterates in the mesh's own copy of the state (the graphs are
-  // bound to it); x_old starts as the same state
+  // bound to it); x starts as the same state
   EG_CUDA(cudaMemcpyAsync(qd, q, 8 * N, mem == EG_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
                           m->stream));
   EG_CUDA(cudaMemcpyAsync(buf, qd, 8 * N, cudaMemcpyDeviceToDevice, m->stream));

@@ -141,7 +141,7 @@ __device__ __forceinline__ void split_element(const DevMesh& md, const double* _
     const double pj = eg::pressure<DIM>(g, qj);
     if (!(qj[0] > 0.0)) atomicOr(status, EG_DEV_NEG_DENSITY);
     if (!(pj > 0.0)) atomicOr(status, EG_DEV_NEG_PRESSURE);
-    nd = eg::ir_node<DIM, false>(g, qj);
+    nd = eg::ir_node<DIM>(g, qj);
     sN[0 * rows + t] = nd.z1;
     sN[1 * rows + t] = nd.zp;
     sN[4 * rows + t] = nd.zu;

@@ -1,7 +1,7 @@
 // eg_static.cu -- eg_rk4 with its scratch in a fixed static device array:
 // the call itself allocates no device or host memory.
 //
-// eg_rk4 takes its six state-sized work vectors from cudaMalloc on its first
+// eg_rk4 takes its four state-sized work vectors from cudaMalloc on its first
 // call on a mesh and keeps them, with the CUDA graphs of its step (whose
 // instantiation may allocate), until the mesh is destroyed or
 // eg_newton_release frees them with cudaFree.  Callers whose device memory is
@@ -11,7 +11,7 @@
 // other streams have in flight.  eg_rk4_static runs the same kernels in the
 // same order (results are bit-identical to eg_rk4), launched one by one, with
 // the work vectors carved from g_rk4_scratch, a file-scope device array of
-// 6 * EG_RK4_STATIC_MAX_DOF doubles (24 MiB) that exists once per device.
+// 4 * EG_RK4_STATIC_MAX_DOF doubles (16 MiB) that exists once per device.
 //
 // Setup: the first call on a device (with that device current) resolves the
 // array's address with cudaGetSymbolAddress, which may load this module;
@@ -34,7 +34,7 @@
 namespace {
 
 constexpr int kMaxDevices = 64;
-constexpr int64_t kScratchDoubles = 6 * (int64_t)EG_RK4_STATIC_MAX_DOF;
+constexpr int64_t kScratchDoubles = 4 * (int64_t)EG_RK4_STATIC_MAX_DOF;
 
 static __device__ __align__(256) double g_rk4_scratch[kScratchDoubles];
 
@@ -124,9 +124,9 @@ extern "C" int eg_rk4_static(eg_mesh* m, double* q, double h, double t_max, int3
   double* buf = nullptr;
   rc = scratch_of_current_device(m, &buf);
   if (rc != EG_OK) return rc;
-  // buf[6][N] = x_old, k1, k2, k3, res, q: the loop iterates in the scratch
+  // buf[4][N] = x, acc, stage state, q: the loop iterates in the scratch
   // copy of the state and writes it back at the end
-  double* qd = buf + 5 * N;
+  double* qd = buf + 3 * N;
   EG_CUDA(cudaMemcpyAsync(qd, q, 8 * N, mem == EG_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
                           m->stream));
   EG_CUDA(cudaMemcpyAsync(buf, qd, 8 * N, cudaMemcpyDeviceToDevice, m->stream));
