@@ -652,11 +652,10 @@ __device__ __forceinline__ T gather(const CoopArgs<T>& a, const BlockView<T>& v,
 // Hessenberg column j and its Givens rotation in R (T, or FP64 for a transposed
 // FP32 solve) by one warp (identical in every block), to the rotations rcs, rsn,
 // the right-hand side rg and the columns rR; h = h1 (+ h2 after a second pass),
-// hn = |w'|.  The j earlier
-// rotations act on the column as the affine recurrence t_0 = h_0, t_{k+1} =
-// -sn_k t_k + cs_k h_{k+1} (row k becomes cs_k t_k + sn_k h_{k+1}), evaluated
-// by a scan over the lanes instead of j dependent steps (the serial form took
-// longer than the apply that it runs beside on small systems).
+// hn = |w'|.  The j earlier rotations act on the column as the affine recurrence
+// t_0 = h_0, t_{k+1} = -sn_k t_k + cs_k h_{k+1} (row k becomes cs_k t_k + sn_k
+// h_{k+1}), evaluated by a scan over the lanes instead of j dependent steps (the
+// serial form took longer than the apply that it runs beside on small systems).
 template <typename R, typename T>
 __device__ __forceinline__ void givens(GmresShared<T>& sm, int j, int M1, int itermax, R* rcs, R* rsn, R* rg, R* rR) {
   const int lane = threadIdx.x & 31;
