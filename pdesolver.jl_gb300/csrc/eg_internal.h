@@ -5,6 +5,7 @@
 
 #include <string>
 
+#include "eg_device_once.h"
 #include "eulergpu.h"
 
 #define EG_MAX_NV 5

@@ -458,15 +458,15 @@ static int launch_element(eg_mesh* m, const double* q, const Epilogue& ep) {
   int st = eg_element_shape(m, epb, mma, &threads, &smem);
   if (st != EG_OK) return st;
   const int blocks = (m->E + epb - 1) / epb;
-  // once per process (thread-safe static initialisation)
-  static const bool attr_set = [] {
+  static EgDeviceOnce once;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  once(dev, [] {
     cudaFuncSetAttribute(k_element<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_element<3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_element<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_element<3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return true;
-  }();
-  (void)attr_set;
+  });
   if (m->dim == 2) {
     if (mma)
       k_element<2, true><<<blocks, threads, smem, m->stream>>>(md, q, m->fflux, ep, m->status, epb);

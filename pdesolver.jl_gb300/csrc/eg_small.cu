@@ -202,12 +202,13 @@ bool eg_small_usable(const eg_mesh* m, const double* q, const Epilogue& ep) {
 }
 
 int eg_launch_small(eg_mesh* m, const double* q, const Epilogue& ep) {
-  static const bool attr_set = [] {
+  static EgDeviceOnce once;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  once(dev, [] {
     cudaFuncSetAttribute(k_small_residual<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_small_residual<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    return true;
-  }();
-  (void)attr_set;
+  });
   const DevMesh md = dev_mesh(m);
   const int epb = small_epb(m), blocks = (m->E + epb - 1) / epb;
   const size_t smem = small_smem(m, epb);

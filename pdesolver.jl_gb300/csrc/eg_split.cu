@@ -247,11 +247,16 @@ __global__ void __launch_bounds__(MAXT) k_split_wide(DevMesh md, const double* _
 template <int DIM>
 int launch_split(eg_mesh* m, const DevMesh& md, const double* q, const Epilogue& ep, int epb, int threads,
                  size_t smem) {
-  // once per process (thread-safe static initialisation)
-  static const int narrow = [] {
+  static EgDeviceOnce once;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  once(dev, [] {
     cudaFuncSetAttribute(k_split_element<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_split_wide<DIM, 768>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     cudaFuncSetAttribute(k_split_wide<DIM, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  });
+  // of the code, the same on every device
+  static const int narrow = [] {
     cudaFuncAttributes a;
     return cudaFuncGetAttributes(&a, k_split_element<DIM>) == cudaSuccess ? a.maxThreadsPerBlock : 0;
   }();
